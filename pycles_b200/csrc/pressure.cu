@@ -19,7 +19,8 @@
 // Thomas and spectral-array traffic, with the same mathematics as the
 // reference's full-spectrum solve.
 //
-//   hmean_partial/hmean_final  HorizontalMean(w), deterministic two-pass sum
+//   hsum_* (plain form)        HorizontalMean(w) in the reference's order
+//   hmean_partial/hmean_final  (precision form) deterministic two-pass sum
 //   (remove_mean_u3)           w -= mean[k] on every cell, applied where w is
 //                              read: in the divergence and in the correction
 //   zero_ghosts                divergence ghosts = 0 (the reference zeroes the
@@ -377,11 +378,9 @@ __global__ void hmean_final(Geo g, const double* __restrict__ partial, double* _
   if (threadIdx.x == 0) mean[k] = red[0] * n_horizontal_i;
 }
 
-// Plain form: HorizontalMean in the reference's order (ParallelMPI.pyx:219-
-// 226).  Each level's sum is one chain of rounded additions over the
-// interior columns, i outer and j inner, which no reordering may change:
-// w's horizontal mean cancels, and the solve subtracts it from every cell.
-// A block owns 32 levels, one lane each.  Warp 0 only adds: it walks a tile
+// The horizontal sums of a field in the reference's order, for callers
+// without scratch memory (pb_horizontal_sums) and for few columns: one chain
+// of rounded additions per level.  A block owns 32 levels, one lane each.  Warp 0 only adds: it walks a tile
 // of kSerialTile columns in shared memory, one dependent addition per column,
 // while the other 31 warps load the next tile (kSerialPer columns each, all
 // loads in flight at once) into the other half of a double buffer.
@@ -434,6 +433,313 @@ __global__ void __launch_bounds__(kSerialWarps * 32, 1) hmean_serial(Geo g, cons
     __syncthreads();
   }
   if (wid == 0 && kok) mean[k] = mul_rn(s, n_horizontal_i);
+}
+
+static int launch_hmean_serial(const Geo& g, const double* w, double* mean, double scale, cudaStream_t st) {
+  const size_t sm = 2 * (size_t)kSerialTile * kSerialLd * sizeof(double);
+  PB_CUDA_TRY(cudaFuncSetAttribute(hmean_serial, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  hmean_serial<<<ceil_div(g.n2, 32), kSerialWarps * 32, sm, st>>>(g, w, mean, scale);
+  pb_note_launch();
+  return PB_OK;
+}
+
+// Plain form: HorizontalMean in the reference's order (ParallelMPI.pyx:219-
+// 226).  Each level's sum is one chain of rounded additions over the
+// interior columns, i outer and j inner, which no reordering may change:
+// w's horizontal mean cancels, and the solve subtracts it from every cell.
+// One lane adding the chain (hmean_serial) is bound by the latency of a
+// dependent FP64 addition, ~20 cycles a column.  Here the chain is cut into
+// segments of about L columns that run side by side, each from a predicted
+// start, and the true sum is moved through their results with the same bits
+// as the chain:
+//
+//   * The prediction p of a segment's start comes from parallel sums of the
+//     columns before it (hsum_parts, hsum_prefix).  It misses the true value
+//     s by some units u in p's last place.
+//   * Two chains of additions of the same columns whose starts differ by a
+//     multiple d of 2 u' (u' the rounding unit of every partial sum they
+//     pass through; the 2 keeps ties to even alike) stay exactly d apart as
+//     long as both are in the same binade after every addition: there the
+//     rounding is a fixed grid.  So kHmChains = 16 chains start at p, p + u,
+//     ..., p + 15u (hsum_chains); s is a multiple of 16u away from one of
+//     them, which covers sums that grow by up to three binades (u' <= 8u),
+//     and the true sum at the segment's end is that chain's end plus s minus
+//     its start (hsum_walk).
+//   * Two more chains start kHmSlack units below and above p.  Rounded
+//     addition is monotone, so a start within kHmSlack / 2 stays between
+//     them; when the two have equal sign and exponent after every addition,
+//     so has everything between.
+//   * Where that does not hold (a sum that starts small and grows, or passes
+//     a power of two or zero within the slack), the walk adds the segment's
+//     columns one by one.  A segment therefore begins at the largest |p|
+//     among the first kHmHead columns around its nominal start: few sums
+//     start small there.  s == p takes the first chain as it is.
+//
+// The walk (one warp per level, ~170 cycles a segment) and the two reads of w
+// bound it.  Measured, FP64 form, one solve: 256x256 columns of 134
+// levels 95 us against 748 for the one-lane chain, 96x96x158 31
+// (108), 64x64x81 21
+// (50).  Segments of 128
+// columns; 64 on grids of up to 8192 columns, where the walk is short and
+// more segments fill the GPU.  Up to 1280 columns hmean_serial stays the
+// faster one (15 us at 32x32 against 20 for the four launches).
+constexpr int kHmChains = 16;
+constexpr int kHmGrow = 3;  // binades a segment's sums may grow by: 2^(kHmGrow + 1) = kHmChains
+constexpr long long kHmSlack = 1 << 14;
+constexpr int kHmHead = 16;
+constexpr int kHmRow = kHmChains + 2;  // a segment's record: the ends, p, flag and bounds
+
+__device__ __forceinline__ double from_bits(long long b) { return __longlong_as_double(b); }
+
+// The interior columns of a level in the reference's order, from column c on.
+struct ColumnWalk {
+  const double* src;
+  long long js, wrap;
+  int j, nl1;
+  __device__ __forceinline__ ColumnWalk(const Geo& g, const double* w, int c, long long k) {
+    nl1 = (int)(g.n1 - 2 * g.gw);
+    const int i = c / nl1;
+    j = c - i * nl1;
+    js = g.js;
+    wrap = g.is - (long long)nl1 * g.js;
+    src = w + (g.gw + i) * g.is + (g.gw + j) * g.js + k;
+  }
+  // the next n columns, +0 (which changes no sum) past the `left` that exist
+  template <int n>
+  __device__ __forceinline__ void take(double (&x)[n], int left) {
+#pragma unroll
+    for (int q = 0; q < n; ++q) {
+      x[q] = q < left ? *src : 0.0;
+      src += js;
+      if (++j == nl1) {
+        j = 0;
+        src += wrap;
+      }
+    }
+  }
+};
+
+// Parallel sum of every nominal segment; a warp takes one segment of 32 levels.
+template <int L>
+__global__ void __launch_bounds__(256) hsum_parts(Geo g, const double* __restrict__ w, double* __restrict__ pre,
+                                                  int nsegs) {
+  const int seg = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const long long k = (long long)blockIdx.y * 32 + (threadIdx.x & 31);
+  if (seg >= nsegs || k >= g.n2) return;
+  const int left = (int)((g.n0 - 2 * g.gw) * (g.n1 - 2 * g.gw)) - seg * L;
+  ColumnWalk cw(g, w, seg * L, k);
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
+  for (int c = 0; c < L; c += 16) {
+    double x[16];
+    cw.take(x, left - c);
+#pragma unroll
+    for (int q = 0; q < 16; ++q) s[q & 3] += x[q];
+  }
+  pre[(long long)seg * g.n2 + k] = (s[0] + s[1]) + (s[2] + s[3]);
+}
+
+// The sums of the segments before each segment, in place: a block takes 32
+// levels, each warp a run of segments.
+__global__ void __launch_bounds__(1024) hsum_prefix(long long n2, double* __restrict__ pre, int nsegs) {
+  __shared__ double run[32][33];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const long long k = (long long)blockIdx.x * 32 + lane;
+  const int per = (nsegs + 31) / 32, s0 = min(w * per, nsegs), s1 = min(s0 + per, nsegs);
+  double t = 0.0;
+  if (k < n2) {
+#pragma unroll 8
+    for (int q = s0; q < s1; ++q) t += pre[q * n2 + k];
+  }
+  run[w][lane] = t;
+  __syncthreads();
+  double before = 0.0;
+  for (int q = 0; q < w; ++q) before += run[q][lane];
+  if (k < n2) {
+#pragma unroll 8
+    for (int q = s0; q < s1; ++q) {
+      const double v = pre[q * n2 + k];
+      pre[q * n2 + k] = before;
+      before += v;
+    }
+  }
+}
+
+// Where a segment begins: after the first b of its nominal columns x, p the
+// prediction there.  (Both segments that meet there evaluate this, on the
+// same values.)
+__device__ __forceinline__ void hm_begin(double& p, int& b, const double (&x)[kHmHead]) {
+  double run = p;
+  b = 0;
+#pragma unroll
+  for (int q = 0; q + 1 < kHmHead; ++q) {
+    run = add_rn(run, x[q]);
+    if (fabs(run) > fabs(p)) {
+      p = run;
+      b = q + 1;
+    }
+  }
+}
+
+template <int L>
+__global__ void __launch_bounds__(64, 8) hsum_chains(Geo g, const double* __restrict__ w,
+                                                      const double* __restrict__ pre, double* __restrict__ rec,
+                                                      int nsegs) {
+  const int seg = blockIdx.x * 2 + (threadIdx.x >> 5);
+  const long long k = (long long)blockIdx.y * 32 + (threadIdx.x & 31);
+  if (seg >= nsegs || k >= g.n2) return;
+  const int left = (int)((g.n0 - 2 * g.gw) * (g.n1 - 2 * g.gw)) - seg * L;
+  ColumnWalk cw(g, w, seg * L, k);
+  double x[kHmHead], y[kHmHead];
+  cw.take(x, left);
+  cw.take(y, left - kHmHead);
+  double p = pre[(long long)seg * g.n2 + k];
+  int b = 0;
+  if (seg > 0) hm_begin(p, b, x);
+  const long long pb = __double_as_longlong(p);
+  double c[kHmChains];
+#pragma unroll
+  for (int r = 0; r < kHmChains; ++r) c[r] = from_bits(pb + r);
+  double lo = from_bits(pb - kHmSlack), hi = from_bits(pb + kHmSlack);
+  int differ = __double2hiint(lo) ^ __double2hiint(hi);
+  int top = 0;  // the largest exponent passed through
+  auto add = [&](double v) {
+#pragma unroll
+    for (int r = 0; r < kHmChains; ++r) c[r] = add_rn(c[r], v);
+    lo = add_rn(lo, v);
+    hi = add_rn(hi, v);
+    differ |= __double2hiint(lo) ^ __double2hiint(hi);
+    top = max(top, __double2hiint(hi) & 0x7fffffff);
+  };
+#pragma unroll
+  for (int q = 0; q < kHmHead; ++q) add(q >= b ? x[q] : 0.0);
+#pragma unroll 1
+  for (int n = kHmHead; n < L; n += kHmHead) {
+    // y holds columns n .. n + 15; the ones after them (the last time: the
+    // next segment's first) are loaded meanwhile
+    cw.take(x, left - n - kHmHead);
+#pragma unroll
+    for (int q = 0; q < kHmHead; ++q) add(y[q]);
+#pragma unroll
+    for (int q = 0; q < kHmHead; ++q) y[q] = x[q];
+  }
+  int bn = 0;
+  if (seg + 1 < nsegs) {
+    double pn = pre[(long long)(seg + 1) * g.n2 + k];
+    hm_begin(pn, bn, y);
+#pragma unroll
+    for (int q = 0; q + 1 < kHmHead; ++q) add(q < bn ? y[q] : 0.0);
+  }
+  const int e0 = (int)(pb >> 52) & 0x7ff;
+  top >>= 20;
+  const long long ok = (differ & 0xfff00000) == 0 && top <= e0 + kHmGrow && top < 0x7fe;
+  double2* row = reinterpret_cast<double2*>(rec + ((long long)k * nsegs + seg) * kHmRow);
+#pragma unroll
+  for (int r = 0; r < kHmChains; r += 2) row[r / 2] = make_double2(c[r], c[r + 1]);
+  row[kHmChains / 2] = make_double2(p, from_bits(ok | (long long)b << 8 | (long long)bn << 16));
+}
+
+// s and the columns c0 .. c1 - 1 of a level, one by one (a warp; out of line,
+// so that the walk's code stays in the instruction cache).
+__device__ __noinline__ double hm_add_columns(double s, const double* w, long long is, long long js, int nl1, int c0,
+                                              int c1) {
+  const int lane = threadIdx.x & 31;
+  for (int cb = c0; cb < c1; cb += 128) {
+    double x[4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const int c = cb + h * 32 + lane;
+      x[h] = c < c1 ? w[c / nl1 * is + c % nl1 * js] : 0.0;
+    }
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      if (cb + h * 32 >= c1) break;
+#pragma unroll
+      for (int m = 0; m < 32; ++m) s = add_rn(s, __shfl_sync(0xffffffffu, x[h], m));
+    }
+  }
+  return s;
+}
+
+// One warp per level moves its sum through the segments, the same in every
+// lane.  The records come through shared memory, kWalkRows at a time, the
+// next ones copied (cp.async) while these are used.
+constexpr int kWalkRows = 32;
+template <int L>
+__global__ void __launch_bounds__(32) hsum_walk(Geo g, const double* __restrict__ w, const double* __restrict__ rec,
+                                                double* __restrict__ mean, double n_horizontal_i, int nsegs) {
+  __shared__ __align__(16) double buf[2][kWalkRows * kHmRow];
+  const int lane = threadIdx.x;
+  const long long k = blockIdx.x;
+  const int ncol = (int)((g.n0 - 2 * g.gw) * (g.n1 - 2 * g.gw));
+  const double* row = rec + (long long)k * nsegs * kHmRow;
+  auto copy = [&](int q0) {  // records q0 .. of the level
+    const int n = min(kWalkRows, nsegs - q0) * kHmRow / 2;  // 16-byte pieces
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(buf[(q0 / kWalkRows) & 1]);
+    for (int e = lane; e < n; e += 32)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + e * 16),
+                   "l"(row + (long long)q0 * kHmRow + 2 * e)
+                   : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  copy(0);
+  double s = 0.0;
+  for (int q0 = 0; q0 < nsegs; q0 += kWalkRows) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+    if (q0 + kWalkRows < nsegs) copy(q0 + kWalkRows);
+    const double* r0 = buf[(q0 / kWalkRows) & 1];
+    const int n = min(kWalkRows, nsegs - q0);
+    for (int q = 0; q < n; ++q) {
+      const double* e = r0 + q * kHmRow;
+      const long long pb = __double_as_longlong(e[kHmChains]);
+      const long long info = __double_as_longlong(e[kHmChains + 1]);
+      const long long d = __double_as_longlong(s) - pb;
+      const int r = (int)d & (kHmChains - 1);
+      const bool near = (info & 1) && (unsigned long long)(d + kHmSlack / 2) <= (unsigned long long)kHmSlack;
+      if (near) {
+        s = add_rn(e[r], sub_rn(s, from_bits(pb + r)));  // the difference: a multiple of 16u
+      } else if (d == 0) {
+        s = e[0];
+      } else {
+        s = hm_add_columns(s, w + g.gw * g.is + g.gw * g.js + k, g.is, g.js, (int)(g.n1 - 2 * g.gw),
+                           (q0 + q) * L + (int)((info >> 8) & 0xff), min((q0 + q + 1) * L + (int)(info >> 16), ncol));
+      }
+    }
+    __syncwarp();
+  }
+  if (lane == 0) mean[k] = mul_rn(s, n_horizontal_i);
+}
+
+template <int L>
+static void launch_hsum(const Geo& g, const double* w, double* mean, double scale, double* scratch, cudaStream_t st) {
+  const long long ncol = (g.n0 - 2 * g.gw) * (g.n1 - 2 * g.gw);
+  const int nsegs = (int)((ncol + L - 1) / L);
+  double* rec = scratch;  // first: 16-byte stores
+  double* pre = scratch + (long long)nsegs * g.n2 * kHmRow;
+  const dim3 grid(ceil_div(nsegs, 8), ceil_div(g.n2, 32));
+  hsum_parts<L><<<grid, 256, 0, st>>>(g, w, pre, nsegs);
+  hsum_prefix<<<ceil_div(g.n2, 32), 1024, 0, st>>>(g.n2, pre, nsegs);
+  hsum_chains<L><<<dim3(ceil_div(nsegs, 2), grid.y), 64, 0, st>>>(g, w, pre, rec, nsegs);
+  hsum_walk<L><<<(unsigned)g.n2, 32, 0, st>>>(g, w, rec, mean, scale, nsegs);
+  for (int q = 0; q < 4; ++q) pb_note_launch();
+}
+
+// scratch: the solve's spectral and Thomas arrays, not yet in use (12 bytes or
+// more per column and interior level; the records and prefixes of segments of
+// 64 columns take at most 9, ghost levels included: 19 doubles for each of
+// at most 1.25 ncol / 64 segments and 3 nz levels).
+static int launch_hmean_ordered(const Geo& g, const double* w, double* mean, double scale, double* scratch,
+                                 cudaStream_t st) {
+  const long long ncol = (g.n0 - 2 * g.gw) * (g.n1 - 2 * g.gw);
+  if (ncol <= 1280) {
+    return launch_hmean_serial(g, w, mean, scale, st);
+  } else if (ncol <= 8192) {
+    launch_hsum<64>(g, w, mean, scale, scratch, st);
+  } else {
+    launch_hsum<128>(g, w, mean, scale, scratch, st);
+  }
+  return PB_OK;
 }
 
 __global__ void zero_ghosts(Geo g, double* __restrict__ f, long long nghost) {
@@ -1128,10 +1434,9 @@ static int pressure_solve_impl(const pb_dims* dims, const double* rho0, const do
   const long long nghost = g.npg - Nx * Ny * nz;
 
   if (precision == PB_FP64) {  // the reference's summation order
-    const size_t sm = 2 * (size_t)kSerialTile * kSerialLd * sizeof(double);
-    PB_CUDA_TRY(cudaFuncSetAttribute(hmean_serial, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    hmean_serial<<<ceil_div(g.n2, 32), kSerialWarps * 32, sm, st>>>(g, w, a.mean, 1.0 / (double)(Ny * Nx));
-    pb_note_launch();
+    const int rc =
+        launch_hmean_ordered(g, w, a.mean, 1.0 / (double)(Ny * Nx), static_cast<double*>(a.spec), st);
+    if (rc) return rc;
   } else {  // precision form: a deterministic parallel sum
     const int kpad = (int)((g.n2 + 31) / 32 * 32);
     hmean_partial<<<kPartials, kpad < 1024 ? kpad : 1024, 0, st>>>(g, w, a.partial);

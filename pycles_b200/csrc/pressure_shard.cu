@@ -77,10 +77,7 @@ extern "C" int pb_horizontal_sums(const pb_dims* dims, const double* field, doub
   if (rc) return rc;
   if (!field || !sums) return PB_ERR_ARG;
   const Geo g = make_geo(dims);
-  const size_t sm = 2 * (size_t)kSerialTile * kSerialLd * sizeof(double);
-  PB_CUDA_TRY(cudaFuncSetAttribute(hmean_serial, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  hmean_serial<<<ceil_div(g.n2, 32), kSerialWarps * 32, sm, as_stream(stream)>>>(g, field, sums, 1.0);
-  pb_note_launch();
+  if ((rc = launch_hmean_serial(g, field, sums, 1.0, as_stream(stream)))) return rc;
   PB_LAUNCH_CHECK();
   return PB_OK;
 }
