@@ -51,6 +51,22 @@ __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
 
+// a / b, correctly rounded, for a divisor used many times: y = 1 / b is
+// formed once (correctly rounded), then q0 = a y misses the quotient by at
+// most two units in the last place, one residual correction makes q1
+// faithful, and a second gives the correctly rounded quotient (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34 (1990): with y correctly rounded and q
+// faithful, fma(fma(-b, q, a), y, q) rounds a / b correctly).  Five
+// operations instead of a division sequence with its range tests.  Needs a
+// quotient and residuals in the normal range (|a| above ~1e-290); a zero,
+// an infinite or a NaN gives zero (its sign may be lost) or NaN.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  const double q0 = __dmul_rn(a, y);
+  const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
+  return __fma_rn(__fma_rn(-b, q1, a), y, q1);
+}
+
 struct Geo {
   long long n0, n1, n2;     // nlg
   long long is, js;         // strides in elements

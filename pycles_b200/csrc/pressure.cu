@@ -44,6 +44,7 @@ namespace {
 
 constexpr int kPartials = 1184;  // 8 x 148 SMs
 constexpr int kFftThreads = 256;  // stockham_pass: nlines * N <= 16 * kFftThreads
+constexpr int kMaxKC = 32;        // levels per x-FFT block at most (two per line, 16 lines)
 
 struct PLayout {
   long long partial, mean, twx, twy, twxf, twyf, kx2, ky2, spec, scr, total;
@@ -758,10 +759,13 @@ constexpr int kDstWrite = 0, kDstAccumulate = 1, kDstDense = 2;
 
 // second_order_divergence (PressureSolver.pyx:138-175, d = 0, 1, 2 in order)
 // of the cell ijk at level k, w taken after remove_mean_u3 (w - mean[k]).
-// Plain form: the reference's divisions by alpha0 in its order, separately
-// rounded; precision form: multiplications by rho0 = 1/alpha0.
+// Plain form: the reference's divisions by alpha0 in its order, each
+// correctly rounded, from the reciprocals 1/alpha0_half[k], 1/alpha0[k] and
+// 1/alpha0[k-1] (yh, yf, yd); precision form: multiplications by
+// rho0 = 1/alpha0.
 template <bool PLAIN>
-__device__ __forceinline__ double divergence_at(const Geo& g, const PArgs& a, long long ijk, long long k) {
+__device__ __forceinline__ double divergence_at(const Geo& g, const PArgs& a, long long ijk, long long k, double yh,
+                                                double yf, double yd) {
   const double* __restrict__ U = a.u;
   const double* __restrict__ V = a.v;
   const double* __restrict__ Wv = a.w;
@@ -770,9 +774,9 @@ __device__ __forceinline__ double divergence_at(const Geo& g, const PArgs& a, lo
   if constexpr (PLAIN) {
     const double ah = a.alpha0_half[k];
     double d = 0.0;
-    d = add_rn(d, mul_rn(sub_rn(U[ijk] / ah, U[ijk - g.is] / ah), g.dxi0));
-    d = add_rn(d, mul_rn(sub_rn(V[ijk] / ah, V[ijk - g.js] / ah), g.dxi1));
-    d = add_rn(d, mul_rn(sub_rn(wc / a.alpha0[k], wm / a.alpha0[k - 1]), g.dxi2));
+    d = add_rn(d, mul_rn(sub_rn(div_by(U[ijk], ah, yh), div_by(U[ijk - g.is], ah, yh)), g.dxi0));
+    d = add_rn(d, mul_rn(sub_rn(div_by(V[ijk], ah, yh), div_by(V[ijk - g.js], ah, yh)), g.dxi1));
+    d = add_rn(d, mul_rn(sub_rn(div_by(wc, a.alpha0[k], yf), div_by(wm, a.alpha0[k - 1], yd)), g.dxi2));
     return d;
   } else {
     const double rh = a.rho0_half[k];
@@ -829,6 +833,14 @@ __global__ void __launch_bounds__(kFftThreads) fft_x_fwd(Geo g, PArgs a, int KCr
   const int ld = line_ld(N);
   const long long ny = g.n1 - 2 * g.gw;
   double* __restrict__ div = a.div;
+  constexpr bool PLAIN = SRC == kSrcDivergence && sizeof(C) == sizeof(double2);
+  // reciprocals of the chunk's alpha0_half and (from the level below on) alpha0
+  __shared__ double yh[PLAIN ? kMaxKC : 1], yf[PLAIN ? kMaxKC + 1 : 1];
+  if constexpr (PLAIN) {
+    if ((int)threadIdx.x < kc) yh[threadIdx.x] = 1.0 / a.alpha0_half[g.gw + k0 + threadIdx.x];
+    if ((int)threadIdx.x <= kc) yf[threadIdx.x] = 1.0 / a.alpha0[g.gw + k0 - 1 + threadIdx.x];
+    __syncthreads();
+  }
 #pragma unroll 4
   for (int e = threadIdx.x; e < N * KC; e += kFftThreads) {
     int kl, il;
@@ -842,7 +854,10 @@ __global__ void __launch_bounds__(kFftThreads) fft_x_fwd(Geo g, PArgs a, int KCr
     const long long ijk = (g.gw + il) * g.is + j * g.js + k;
     double d;
     if constexpr (SRC == kSrcDivergence) {
-      d = divergence_at<sizeof(C) == sizeof(double2)>(g, a, ijk, k);
+      if constexpr (PLAIN)
+        d = divergence_at<true>(g, a, ijk, k, yh[kl], yf[kl + 1], yf[kl]);
+      else
+        d = divergence_at<false>(g, a, ijk, k, 0.0, 0.0, 0.0);
       div[ijk] = d;
     } else if constexpr (SRC == kSrcResidual) {
       d = residual_at(g, a, ijk, k, k - g.gw, nz);
