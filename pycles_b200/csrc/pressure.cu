@@ -317,6 +317,96 @@ template <class C> __device__ __forceinline__ const C* twy_of(const PArgs& a);
 template <> __device__ __forceinline__ const double2* twy_of<double2>(const PArgs& a) { return a.twy; }
 template <> __device__ __forceinline__ const float2* twy_of<float2>(const PArgs& a) { return a.twyf; }
 
+// ---- line FFTs of compile-time lengths 2^LG, LG = 5 .. 10 --------------------
+// LINES lines in shared memory, LINES N / 8 threads, one radix-8 item (8
+// values) per thread.  64 registers a thread at 512 threads keep 1024 threads
+// on an SM in FP64, twice what 16 values per thread allowed, and these
+// kernels are bound by the latency of their loads and of the passes.  The
+// first pass takes its inputs and the last one leaves its results where the
+// kernel says (global memory for the y-FFTs and the inverse x-FFT), so a
+// line crosses shared memory once per pass instead of twice.  Measured at
+// 256x256x128, FP64: forward x-FFT 155 -> 108 us, y-FFTs 63 and 53 -> 33 and
+// 29, inverse x-FFT 67 -> 49; FP32 at 512x512x256: y-FFT 240 -> 150.
+// Line stride: consecutive threads take consecutive lines at one position
+// (8 of 16 bytes or 16 of 8 bytes make a phase of a shared-memory access), so
+// the stride is odd where a phase holds one position and 2 or 4 where it
+// holds 2 or 4 consecutive ones: free of bank conflicts.
+template <class C, int LG>
+struct Ct {
+  static constexpr int N = 1 << LG;
+  static constexpr int LINES = ct_lines(LG);
+  static constexpr int LGL = LINES == 16 ? 4 : (LINES == 8 ? 3 : 2);
+  static constexpr int NT = LINES * N / 8;
+  static constexpr int PHASE = 128 / (int)sizeof(C);
+  static constexpr int LD = N + N / 8 + (LINES >= PHASE ? 1 : PHASE / LINES);
+  static constexpr int LGLAST = LG % 3 == 0 ? 3 : LG % 3;  // radix of the last pass (radix 8 before it)
+  static constexpr size_t SMEM = (size_t)LINES * LD * sizeof(C);
+  static __device__ __forceinline__ int at(int l, int x) { return l * LD + swz(x); }
+};
+
+// One radix-2^LGR pass of the Stockham FFT after LGNS bits are done: load(l,
+// x, r) gives input x of line l, store(l, x, value) takes output x; SYNC: a
+// barrier between the last load and the first store (both in the buffer).
+// LFAST: consecutive threads take consecutive lines, else positions.
+template <class C, int LG, int LGR, int LGNS, bool SYNC, bool LFAST, class Load, class Store>
+__device__ __forceinline__ void ct_pass(const C* __restrict__ tw, bool inverse, Load load, Store store) {
+  using T = Ct<C, LG>;
+  constexpr int R = 1 << LGR, IT = 8 / R, LGPER = LG - LGR;
+  C v[IT][R];
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    const int b = threadIdx.x + it * T::NT;
+    const int l = LFAST ? b & (T::LINES - 1) : b >> LGPER;
+    const int j = LFAST ? b >> T::LGL : b & ((1 << LGPER) - 1);
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[it][r] = load(l, j + (r << LGPER));
+    if constexpr (LGNS > 0) {
+      const int k = j & ((1 << LGNS) - 1);
+#pragma unroll
+      for (int r = 1; r < R; ++r) {
+        C w = tw[(k * r) << (LG - LGNS - LGR)];
+        if (inverse) w.y = -w.y;
+        v[it][r] = cmul(v[it][r], w);
+      }
+    }
+    if constexpr (R == 8) dft8(v[it], inverse);
+    else if constexpr (R == 4) dft4(v[it][0], v[it][1], v[it][2], v[it][3], inverse);
+    else dft2(v[it]);
+  }
+  if constexpr (SYNC) __syncthreads();
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    const int b = threadIdx.x + it * T::NT;
+    const int l = LFAST ? b & (T::LINES - 1) : b >> LGPER;
+    const int j = LFAST ? b >> T::LGL : b & ((1 << LGPER) - 1);
+    const int k = j & ((1 << LGNS) - 1);
+    const int base = ((j - k) << LGR) + k;
+#pragma unroll
+    for (int r = 0; r < R; ++r) store(l, base + (r << LGNS), v[it][r]);
+  }
+}
+
+// All passes: the first from `load`, the last to `store` (TO_BUF: into the
+// buffer itself).  The buffer must be free when it is called (FROM_BUF: hold
+// the input, synchronised).
+template <class C, int LG, bool FROM_BUF, bool TO_BUF, bool LFAST1, class Load, class Store>
+__device__ __forceinline__ void ct_fft(C* buf, const C* __restrict__ tw, bool inverse, Load load, Store store) {
+  using T = Ct<C, LG>;
+  auto get = [&](int l, int x) { return buf[T::at(l, x)]; };
+  auto put = [&](int l, int x, C v) { buf[T::at(l, x)] = v; };
+  ct_pass<C, LG, 3, 0, FROM_BUF, LFAST1>(tw, inverse, load, put);
+  __syncthreads();
+  if constexpr (LG >= 7) {
+    ct_pass<C, LG, 3, 3, true, true>(tw, inverse, get, put);
+    __syncthreads();
+  }
+  if constexpr (LG == 10) {
+    ct_pass<C, LG, 3, 6, true, true>(tw, inverse, get, put);
+    __syncthreads();
+  }
+  ct_pass<C, LG, T::LGLAST, LG - T::LGLAST, TO_BUF, true>(tw, inverse, get, store);
+}
+
 // ---- HorizontalMean (ParallelMPI.pyx:196-241) ------------------------------
 // Block b sums a contiguous chunk of interior columns for every level (one
 // thread per level, four interleaved accumulators for memory-level
@@ -811,11 +901,22 @@ __device__ __forceinline__ double residual_at(const Geo& g, const PArgs& a, long
 // SRC = kSrcDense: the right-hand side is read from a dense interior array
 //   (a slab of levels of a sharded solve).
 //
-// LGN > 0 instantiates the kernel for N = 2^LGN (KC = 2 ct_lines(LGN)), so
-// that the index arithmetic and the FFT passes are compile-time; LGN = 0
-// takes N and KC at run time.
+// LGN > 0 instantiates the kernel for N = 2^LGN (KC = 2 ct_lines(LGN)), with
+// the compile-time transform; LGN = 0 takes N and KC at run time.
+template <class C, int LGN>
+__host__ __device__ constexpr int fft_threads() {
+  if constexpr (LGN > 0) return Ct<C, LGN>::NT;
+  return kFftThreads;
+}
+// resident blocks per SM the registers are held to: blocks of 512
+// threads run two to an SM
+template <class C, int LGN>
+constexpr int fft_blocks() {
+  return LGN >= 8 ? 2 : 1;
+}
+
 template <class C, int SRC, int LGN>
-__global__ void __launch_bounds__(kFftThreads) fft_x_fwd(Geo g, PArgs a, int KCrt) {
+__global__ void __launch_bounds__((fft_threads<C, LGN>()), (fft_blocks<C, LGN>())) fft_x_fwd(Geo g, PArgs a, int KCrt) {
   using R = decltype(C().x);
   constexpr bool CT = LGN > 0;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -830,7 +931,8 @@ __global__ void __launch_bounds__(kFftThreads) fft_x_fwd(Geo g, PArgs a, int KCr
   const int kc = min(KC, nz - k0);
   const int lc = (kc + 1) >> 1;
   const long long j = g.gw + jl;
-  const int ld = line_ld(N);
+  constexpr int NT = fft_threads<C, LGN>();
+  const int ld = CT ? Ct<C, CT ? LGN : 5>::LD : line_ld(N);
   const long long ny = g.n1 - 2 * g.gw;
   double* __restrict__ div = a.div;
   constexpr bool PLAIN = SRC == kSrcDivergence && sizeof(C) == sizeof(double2);
@@ -842,7 +944,7 @@ __global__ void __launch_bounds__(kFftThreads) fft_x_fwd(Geo g, PArgs a, int KCr
     __syncthreads();
   }
 #pragma unroll 4
-  for (int e = threadIdx.x; e < N * KC; e += kFftThreads) {
+  for (int e = threadIdx.x; e < N * KC; e += NT) {
     int kl, il;
     split_idx(e, KC, il, kl);
     const int slot = 2 * ((kl >> 1) * ld + swz(il)) + (kl & 1);
@@ -867,13 +969,21 @@ __global__ void __launch_bounds__(kFftThreads) fft_x_fwd(Geo g, PArgs a, int KCr
     inr[slot] = (R)d;
   }
   __syncthreads();
-  const C* res = fft_lines<C>(in, CT ? (KC >> 1) : lc, KC >> 1, N, twx_of<C>(a), false);
+  const C* res = in;
+  if constexpr (CT) {
+    using T = Ct<C, LGN>;
+    ct_fft<C, LGN, true, true, true>(in, twx_of<C>(a), false, [&](int l, int x) { return in[T::at(l, x)]; },
+                                     [&](int l, int x, C v) { in[T::at(l, x)] = v; });
+    __syncthreads();
+  } else {
+    res = fft_lines<C>(in, lc, KC >> 1, N, twx_of<C>(a), false);
+  }
   // separate the two rows of each line; write the columns m = 0..N/2
   C* spec = reinterpret_cast<C*>(a.spec);
   const long long nxy = (long long)Nh * (g.n1 - 2 * g.gw);
   const R half = (R)0.5;
 #pragma unroll 4
-  for (int e = threadIdx.x; e < Nh * kc; e += kFftThreads) {
+  for (int e = threadIdx.x; e < Nh * kc; e += NT) {
     const int kl = e / Nh;
     const int m = e - kl * Nh;
     const C* line = res + (kl >> 1) * ld;
@@ -894,14 +1004,29 @@ __global__ void __launch_bounds__(kFftThreads) fft_x_fwd(Geo g, PArgs a, int KCr
 // ---- y-FFT over W[k][j][m] lines along j, IC columns m per block ----------
 // (LGN as for fft_x_fwd: N = 2^LGN and IC = ct_lines(LGN) at compile time.)
 template <class C, bool INV, int LGN>
-__global__ void __launch_bounds__(kFftThreads) fft_y(Geo g, PArgs a, int ICrt) {
-  constexpr bool CT = LGN > 0;
+__global__ void __launch_bounds__((fft_threads<C, LGN>()), (fft_blocks<C, LGN>())) fft_y(Geo g, PArgs a, int ICrt) {
   extern __shared__ __align__(16) unsigned char smraw[];
   C* in = reinterpret_cast<C*>(smraw);
   const int Nx = (int)(g.n0 - 2 * g.gw) / 2 + 1;  // stored x-modes
-  const int N = CT ? (1 << LGN) : (int)(g.n1 - 2 * g.gw);
-  const int IC = CT ? ct_lines(LGN) : ICrt;
   const int kk = blockIdx.y;
+  if constexpr (LGN > 0) {
+    using T = Ct<C, LGN>;
+    const int i0 = blockIdx.x * T::LINES, ic = Nx - i0;
+    C* plane = reinterpret_cast<C*>(a.spec) + (long long)kk * T::N * Nx + i0;
+    const double sc = INV ? 1.0 / (double)T::N : 1.0;
+    ct_fft<C, LGN, false, false, true>(
+        in, twy_of<C>(a), INV, [&](int l, int x) { return l < ic ? plane[x * Nx + l] : czero<C>(); },
+        [&](int l, int x, C r) {
+          if (INV) {
+            r.x *= sc;
+            r.y *= sc;
+          }
+          if (l < ic) plane[x * Nx + l] = r;
+        });
+    return;
+  }
+  const int N = (int)(g.n1 - 2 * g.gw);
+  const int IC = ICrt;
   const int i0 = blockIdx.x * IC;
   const int ic = min(IC, Nx - i0);
   const int ld = line_ld(N);
@@ -914,7 +1039,7 @@ __global__ void __launch_bounds__(kFftThreads) fft_y(Geo g, PArgs a, int ICrt) {
     in[il * ld + swz(jl)] = plane[(long long)jl * Nx + i0 + il];
   }
   __syncthreads();
-  const C* res = fft_lines<C>(in, CT ? IC : ic, IC, N, twy_of<C>(a), INV);
+  const C* res = fft_lines<C>(in, ic, IC, N, twy_of<C>(a), INV);
   const double sc = INV ? 1.0 / (double)N : 1.0;
 #pragma unroll 4
   for (int e = threadIdx.x; e < N * IC; e += kFftThreads) {
@@ -1067,22 +1192,78 @@ __global__ void __launch_bounds__(256, sizeof(C) == 8 ? 4 : 2) tdma_kernel(Geo g
 // two real rows as Re z and Im z.
 // (LGN as for fft_x_fwd.)
 template <class C, int DST, int LGN>
-__global__ void __launch_bounds__(kFftThreads) fft_x_inv(Geo g, PArgs a, int KCrt) {
+__global__ void __launch_bounds__((fft_threads<C, LGN>()), (fft_blocks<C, LGN>())) fft_x_inv(Geo g, PArgs a, int KCrt) {
   constexpr bool ACC = DST == kDstAccumulate;
-  constexpr bool CT = LGN > 0;
   extern __shared__ __align__(16) unsigned char smraw[];
   C* in = reinterpret_cast<C*>(smraw);
-  const int N = CT ? (1 << LGN) : (int)(g.n0 - 2 * g.gw);
-  const int KC = CT ? 2 * ct_lines(LGN) : KCrt;
+  const int N = LGN > 0 ? (1 << LGN) : (int)(g.n0 - 2 * g.gw);
+  const int KC = LGN > 0 ? 2 * ct_lines(LGN) : KCrt;
   const int Nh = N / 2 + 1;
   const int nz = (int)(g.n2 - 2 * g.gw);
   const int jl = blockIdx.x;
   const int k0 = blockIdx.y * KC;
   const int kc = min(KC, nz - k0);
   const int lc = (kc + 1) >> 1;
-  const int ld = line_ld(N);
   const C* spec = reinterpret_cast<const C*>(a.spec);
-  const long long nxy = (long long)Nh * (g.n1 - 2 * g.gw);
+  const long long ny = g.n1 - 2 * g.gw;
+  const long long nxy = (long long)Nh * ny;
+  const double sc = 1.0 / (double)N;
+  // where the value of x position il and level k0 + kl goes
+  double* __restrict__ out = DST == kDstDense ? a.dst_dense + (long long)jl * nz + k0
+                                              : a.p + g.gw * g.is + (g.gw + jl) * g.js + g.gw + k0;
+  const long long so = DST == kDstDense ? ny * nz : g.is;
+  if constexpr (LGN > 0) {
+    // Z[m] = A[m] + i B[m], and for m > N/2 conj A[N-m] + i conj B[N-m]
+    using T = Ct<C, LGN>;
+    const C* row = spec + (long long)k0 * nxy + (long long)jl * Nh;
+    auto load = [&](int l, int x) {
+      C z = czero<C>();
+      if (l < lc) {
+        const bool up = x > N / 2;
+        const C* src = row + (long long)(2 * l) * nxy + (up ? N - x : x);
+        const C A = src[0];
+        const C B = 2 * l + 1 < kc ? src[nxy] : czero<C>();
+        z.x = up ? A.x + B.y : A.x - B.y;
+        z.y = up ? B.x - A.y : A.y + B.x;
+      }
+      return z;
+    };
+    auto store = [&](int l, int x, C z) {
+      double* dst = out + x * so + 2 * l;
+      const double x0 = (double)z.x * sc, x1 = (double)z.y * sc;
+      if (2 * l < kc) dst[0] = ACC ? dst[0] + x0 : x0;
+      if (2 * l + 1 < kc) dst[1] = ACC ? dst[1] + x1 : x1;
+    };
+    if constexpr (sizeof(C) == 16) {
+      ct_fft<C, LGN, false, false, false>(in, twx_of<C>(a), true, load, store);
+    } else {
+      // FP32: the stores of the last pass, two levels a thread, would be half
+      // of the kernel's accesses; through the buffer consecutive threads write
+      // consecutive levels
+      ct_fft<C, LGN, false, true, false>(in, twx_of<C>(a), true, load,
+                                         [&](int l, int x, C z) { in[T::at(l, x)] = z; });
+      __syncthreads();
+      constexpr int kBatch = 4;  // the pressure loads of a batch are issued before its stores
+#pragma unroll 1
+      for (int e0 = threadIdx.x; e0 < N * KC; e0 += kBatch * T::NT) {
+        double val[kBatch], old[kBatch];
+#pragma unroll
+        for (int h = 0; h < kBatch; ++h) {
+          const int e = e0 + h * T::NT, il = e / KC, kl = e % KC;
+          const C z = in[T::at(kl >> 1, il)];
+          val[h] = (double)((kl & 1) ? z.y : z.x) * sc;
+          old[h] = ACC && kl < kc ? out[il * so + kl] : 0.0;
+        }
+#pragma unroll
+        for (int h = 0; h < kBatch; ++h) {
+          const int e = e0 + h * T::NT, il = e / KC, kl = e % KC;
+          if (kl < kc) out[il * so + kl] = ACC ? old[h] + val[h] : val[h];
+        }
+      }
+    }
+    return;
+  }
+  const int ld = line_ld(N);
 #pragma unroll 4
   for (int e = threadIdx.x; e < Nh * lc; e += kFftThreads) {
     const int p = e / Nh;
@@ -1103,43 +1284,15 @@ __global__ void __launch_bounds__(kFftThreads) fft_x_inv(Geo g, PArgs a, int KCr
     }
   }
   __syncthreads();
-  const C* res = fft_lines<C>(in, CT ? (KC >> 1) : lc, KC >> 1, N, twx_of<C>(a), true);
-  const double sc = 1.0 / (double)N;
-  const long long j = g.gw + jl;
-  double* __restrict__ p = a.p;
-  if constexpr (DST == kDstDense) {
-    const long long ny = g.n1 - 2 * g.gw;
-    for (int e = threadIdx.x; e < N * KC; e += kFftThreads) {
-      int kl = 0, il = 0;
-      split_idx(e, KC, il, kl);
-      if (kl >= kc) continue;
-      const C z = res[(kl >> 1) * ld + swz(il)];
-      a.dst_dense[((long long)il * ny + jl) * nz + k0 + kl] = (double)((kl & 1) ? z.y : z.x) * sc;
-    }
-    return;
-  }
-  // batches of kBatch elements: the pressure loads of a batch (ACC) are all
-  // issued before its stores
-  constexpr int kBatch = 8;
-  for (int e0 = threadIdx.x; e0 < N * KC; e0 += kBatch * kFftThreads) {
-    long long ijk[kBatch];
-    double val[kBatch], old[kBatch];
-#pragma unroll
-    for (int b = 0; b < kBatch; ++b) {
-      const int e = e0 + b * kFftThreads;
-      int kl = 0, il = 0;
-      split_idx(e, KC, il, kl);
-      const bool ok = e < N * KC && kl < kc;
-      ijk[b] = ok ? (g.gw + il) * g.is + j * g.js + g.gw + k0 + kl : -1;
-      if (ok) {
-        const C z = res[(kl >> 1) * ld + swz(il)];
-        val[b] = (double)((kl & 1) ? z.y : z.x) * sc;
-      }
-      old[b] = (ACC && ok) ? p[ijk[b]] : 0.0;
-    }
-#pragma unroll
-    for (int b = 0; b < kBatch; ++b)
-      if (ijk[b] >= 0) p[ijk[b]] = ACC ? old[b] + val[b] : val[b];
+  const C* res = fft_lines<C>(in, lc, KC >> 1, N, twx_of<C>(a), true);
+#pragma unroll 4
+  for (int e = threadIdx.x; e < N * KC; e += kFftThreads) {
+    int kl = 0, il = 0;
+    split_idx(e, KC, il, kl);
+    if (kl >= kc) continue;
+    const C z = res[(kl >> 1) * ld + swz(il)];
+    const double x = mul_rn((double)((kl & 1) ? z.y : z.x), sc);
+    out[il * so + kl] = ACC ? add_rn(out[il * so + kl], x) : x;
   }
 }
 
@@ -1268,9 +1421,9 @@ extern "C" int pb_pressure_init(const pb_dims* dims, void* workspace, long long 
   return PB_OK;
 }
 
-// log2 of a length that has compile-time FFT kernels (128 ... 1024), else 0
+// log2 of a length that has compile-time FFT kernels (32 ... 1024), else 0
 int ct_lg(long long n) {
-  if (!pow2(n) || n < 128 || n > 1024) return 0;
+  if (!pow2(n) || n < 32 || n > 1024) return 0;
   int lg = 0;
   while ((1LL << lg) < n) ++lg;
   return lg;
@@ -1280,7 +1433,7 @@ template <class C, int SRC, int LG>
 static int launch_x_fwd_src(const Geo& g, PArgs& a, dim3 grid, size_t sm, int KC, cudaStream_t st) {
   if (sm > 48 * 1024)
     PB_CUDA_TRY(cudaFuncSetAttribute(fft_x_fwd<C, SRC, LG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  fft_x_fwd<C, SRC, LG><<<grid, kFftThreads, sm, st>>>(g, a, KC);
+  fft_x_fwd<C, SRC, LG><<<grid, fft_threads<C, LG>(), sm, st>>>(g, a, KC);
   return PB_OK;
 }
 
@@ -1297,7 +1450,7 @@ template <class C, int DST, int LG>
 static int launch_x_inv_dst(const Geo& g, PArgs& a, dim3 grid, size_t sm, int KC, cudaStream_t st) {
   if (sm > 48 * 1024)
     PB_CUDA_TRY(cudaFuncSetAttribute(fft_x_inv<C, DST, LG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  fft_x_inv<C, DST, LG><<<grid, kFftThreads, sm, st>>>(g, a, KC);
+  fft_x_inv<C, DST, LG><<<grid, fft_threads<C, LG>(), sm, st>>>(g, a, KC);
   return PB_OK;
 }
 
@@ -1317,21 +1470,30 @@ static int launch_y(const Geo& g, PArgs& a, bool inverse, dim3 grid, size_t sm, 
     PB_CUDA_TRY(cudaFuncSetAttribute(fft_y<C, true, LG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   }
   if (inverse)
-    fft_y<C, true, LG><<<grid, kFftThreads, sm, st>>>(g, a, IC);
+    fft_y<C, true, LG><<<grid, fft_threads<C, LG>(), sm, st>>>(g, a, IC);
   else
-    fft_y<C, false, LG><<<grid, kFftThreads, sm, st>>>(g, a, IC);
+    fft_y<C, false, LG><<<grid, fft_threads<C, LG>(), sm, st>>>(g, a, IC);
   return PB_OK;
 }
 
 // Dispatch on a length's compile-time instantiation (LG = 0: run-time length).
 #define PB_FFT_DISPATCH(lg, call)         \
   switch (lg) {                           \
+    case 5: { constexpr int L_ = 5; call; } break;   \
+    case 6: { constexpr int L_ = 6; call; } break;   \
     case 7: { constexpr int L_ = 7; call; } break;   \
     case 8: { constexpr int L_ = 8; call; } break;   \
     case 9: { constexpr int L_ = 9; call; } break;   \
     case 10: { constexpr int L_ = 10; call; } break; \
     default: { constexpr int L_ = 0; call; } break;  \
   }
+
+template <class C>
+static size_t ct_smem(int lg) {
+  size_t sm = 0;
+  PB_FFT_DISPATCH(lg, sm = (Ct<C, (L_ > 0 ? L_ : 5)>::SMEM));
+  return sm;
+}
 
 // The spectral solve in phases, so that a sharded solve can exchange data
 // between them: (1) forward x-FFT (from src) and forward y-FFT of every level
@@ -1350,14 +1512,13 @@ static int fft_shape(const Geo& g, FftShape& f) {
   f.Ny = g.n1 - 2 * g.gw;
   f.nz = g.n2 - 2 * g.gw;
   f.Nh = f.Nx / 2 + 1;  // stored x-modes
-  f.LC = lines_for(f.Nx, sizeof(C));  // complex lines per x-FFT block
-  f.KC = 2 * f.LC;                    // levels per x-FFT block (two per line)
-  f.smx = fft_smem(f.Nx, f.LC, sizeof(C));
-  f.IC = lines_for(f.Ny, sizeof(C));
-  f.smy = fft_smem(f.Ny, f.IC, sizeof(C));
   f.lgx = ct_lg(f.Nx);
   f.lgy = ct_lg(f.Ny);
-  if ((f.lgx && f.LC != ct_lines(f.lgx)) || (f.lgy && f.IC != ct_lines(f.lgy))) return PB_ERR_UNSUPPORTED;
+  f.LC = f.lgx ? ct_lines(f.lgx) : lines_for(f.Nx, sizeof(C));  // complex lines per x-FFT block
+  f.KC = 2 * f.LC;                                               // levels per x-FFT block (two per line)
+  f.smx = f.lgx ? ct_smem<C>(f.lgx) : fft_smem(f.Nx, f.LC, sizeof(C));
+  f.IC = f.lgy ? ct_lines(f.lgy) : lines_for(f.Ny, sizeof(C));
+  f.smy = f.lgy ? ct_smem<C>(f.lgy) : fft_smem(f.Ny, f.IC, sizeof(C));
   f.gx = dim3((unsigned)f.Ny, ceil_div(f.nz, f.KC));
   f.gy = dim3(ceil_div(f.Nh, f.IC), (unsigned)f.nz);
   return PB_OK;
