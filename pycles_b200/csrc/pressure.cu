@@ -109,7 +109,8 @@ template <> __device__ __forceinline__ float2 creal<float2>(double x) { return m
 // accesses fall on distinct bank pairs; other lengths take an odd stride.
 __host__ __device__ __forceinline__ int line_ld(int N) {
   const int base = N + N / 8;
-  if ((N & (N - 1)) != 0 || N < 256) return base + 1;
+  if ((N & (N - 1)) != 0) return base | 1;
+  if (N < 256) return base + 1;
   const int want = (N / 256) & 15;  // 16 / IC mod 16
   return base + ((want - base % 16) + 16) % 16;
 }
@@ -246,39 +247,137 @@ __device__ __forceinline__ void split_idx(int e, int d, int& q, int& r) {
   }
 }
 
-// Direct DFT for lengths that are not powers of two: out = DFT(in), both in
-// the swizzled line layout.
-template <class C>
-__device__ void dft_lines(const C* in, C* out, int nlines, int N, const C* __restrict__ tw, bool inverse) {
-  const int ld = line_ld(N);
-  for (int e = threadIdx.x; e < nlines * N; e += kFftThreads) {
-    const int line = e / N;
-    const int m = e - line * N;
-    C acc = czero<C>();
-    const C* x = in + line * ld;
-    int idx = 0;
-    for (int n = 0; n < N; ++n) {
-      C w = tw[idx];
-      if (inverse) w.y = -w.y;
-      acc = cadd(acc, cmul(w, x[swz(n)]));
-      idx += m;
-      if (idx >= N) idx -= N;
-    }
-    out[line * ld + swz(m)] = acc;
+// Lengths that are not powers of two: direct sums out[m] = sum_n w^(mn)
+// in[n], n ascending, both line sets in the swizzled layout.  A thread takes
+// TM outputs of one line, m = m0 + q G, so that one input load serves TM
+// products and consecutive threads read consecutive lines at one position
+// with the same twiddles (broadcasts); the twiddles are staged in shared
+// memory, conjugated for the inverse.  One output per thread, with its own
+// input and global twiddle loads and index, ran at a tenth of the FP64 pipe.
+// Measured, one y-FFT: 36 us at 96x96x150 (FP64; 113 before), 37 at
+// 150x120x90 (FP32; 105 before).
+__device__ __forceinline__ double mul_add(double a, double b, double c, double d, double acc) {  // acc + (a b + c d)
+  return __dadd_rn(acc, __fma_rn(a, b, __dmul_rn(c, d)));
+}
+__device__ __forceinline__ float mul_add(float a, float b, float c, float d, float acc) {
+  return __fadd_rn(acc, __fmaf_rn(a, b, __fmul_rn(c, d)));
+}
+// acc + w x, each product's rounding as it always was, the two directions' too
+template <class C, bool INV>
+__device__ __forceinline__ void dft_term(C& acc, C w, C x) {
+  acc.x = mul_add(w.x, x.x, -w.y, x.y, acc.x);
+  acc.y = INV ? mul_add(w.x, x.y, w.y, x.x, acc.y) : mul_add(w.y, x.x, w.x, x.y, acc.y);
+}
+
+// N = TM G: with n = n0 + r, n0 a multiple of TM, the twiddle of output q is
+// number m0 n + G (q r mod TM) mod N.  The table holds row[b][c] = number
+// b + G c, so the TM twiddles of an input are one row, and which output takes
+// which is known at compile time: the index is one step per input instead of
+// one per product.
+template <class C, int TM, bool INV>
+__device__ __forceinline__ void dft_rows(const C* in, C* out, C* table, int nlines, int N, const C* __restrict__ tw) {
+  const int ld = line_ld(N), G = N / TM;
+  for (int e = threadIdx.x; e < N * TM; e += kFftThreads) {
+    const int b = e / TM, m = b + (e - b * TM) * G;
+    C w = tw[m < N ? m : m - N];
+    if (INV) w.y = -w.y;
+    table[e] = w;
   }
   __syncthreads();
+  for (int e = threadIdx.x; e < nlines * G; e += kFftThreads) {
+    const int m0 = e / nlines, l = e - m0 * nlines;
+    C acc[TM];
+#pragma unroll
+    for (int q = 0; q < TM; ++q) acc[q] = czero<C>();
+    const C* line = in + l * ld;
+    int b = 0;
+    for (int n0 = 0; n0 < N; n0 += TM) {
+#pragma unroll
+      for (int r = 0; r < TM; ++r) {
+        const C x = line[swz(n0 + r)];
+        C w[TM];
+#pragma unroll
+        for (int c = 0; c < TM; ++c) w[c] = table[b * TM + c];
+#pragma unroll
+        for (int q = 0; q < TM; ++q) dft_term<C, INV>(acc[q], w[(q * r) % TM], x);
+        b += m0;
+        if (b >= N) b -= N;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < TM; ++q) out[l * ld + swz(m0 + q * G)] = acc[q];
+  }
+  __syncthreads();
+}
+
+// Any N: G = N / TM rounded up, an index per output.
+template <class C, bool INV>
+__device__ __forceinline__ void dft_any(const C* in, C* out, C* stw, int nlines, int N, const C* __restrict__ tw) {
+  constexpr int TM = 6;
+  const int ld = line_ld(N), G = (N + TM - 1) / TM;
+  for (int m = threadIdx.x; m < N; m += kFftThreads) {
+    C w = tw[m];
+    if (INV) w.y = -w.y;
+    stw[m] = w;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < nlines * G; e += kFftThreads) {
+    const int m0 = e / nlines, l = e - m0 * nlines;
+    C acc[TM];
+    int idx[TM];
+#pragma unroll
+    for (int q = 0; q < TM; ++q) {
+      acc[q] = czero<C>();
+      idx[q] = 0;
+    }
+    const C* line = in + l * ld;
+#pragma unroll 4
+    for (int n = 0; n < N; ++n) {
+      const C x = line[swz(n)];
+#pragma unroll
+      for (int q = 0; q < TM; ++q) {
+        dft_term<C, INV>(acc[q], stw[idx[q]], x);
+        // an output past the last, m = m0 + q G >= N, only keeps its index
+        // in range: m < N + TM, so two steps back always do
+        idx[q] += m0 + q * G;
+        if (idx[q] >= N) idx[q] -= N;
+        if (idx[q] >= N) idx[q] -= N;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < TM; ++q) {
+      const int m = m0 + q * G;
+      if (m < N) out[l * ld + swz(m)] = acc[q];
+    }
+  }
+  __syncthreads();
+}
+
+template <class C, bool INV>
+__device__ __forceinline__ void dft_lines(const C* in, C* out, C* table, int nlines, int N, int tm,
+                                          const C* __restrict__ tw) {
+  switch (tm) {
+    case 4: dft_rows<C, 4, INV>(in, out, table, nlines, N, tw); break;
+    case 5: dft_rows<C, 5, INV>(in, out, table, nlines, N, tw); break;
+    case 6: dft_rows<C, 6, INV>(in, out, table, nlines, N, tw); break;
+    case 8: dft_rows<C, 8, INV>(in, out, table, nlines, N, tw); break;
+    case 10: dft_rows<C, 10, INV>(in, out, table, nlines, N, tw); break;
+    default: dft_any<C, INV>(in, out, table, nlines, N, tw); break;
+  }
 }
 
 // Transform the lines in `in`; returns where the result is.
 template <class C>
 __device__ __forceinline__ C* fft_lines(C* in, int nlines, int maxlines, int N, const C* __restrict__ tw,
-                                        bool inverse) {
+                                        int tm, bool inverse) {
   if (is_pow2(N)) {
     fft_lines_pow2<C>(in, nlines, N, tw, inverse);
     return in;
   }
   C* out = in + (size_t)maxlines * line_ld(N);
-  dft_lines<C>(in, out, nlines, N, tw, inverse);
+  C* table = out + (size_t)maxlines * line_ld(N);
+  if (inverse) dft_lines<C, true>(in, out, table, nlines, N, tm, tw);
+  else dft_lines<C, false>(in, out, table, nlines, N, tm, tw);
   return out;
 }
 
@@ -308,6 +407,7 @@ struct PArgs {
   const double* src_dense;
   double* dst_dense;
   int j0;
+  int tmx, tmy;  // outputs per thread of a direct transform along x and y (direct_outputs)
 };
 
 template <class C> __device__ __forceinline__ const C* twx_of(const PArgs& a);
@@ -909,9 +1009,11 @@ __host__ __device__ constexpr int fft_threads() {
   return kFftThreads;
 }
 // resident blocks per SM the registers are held to: blocks of 512
-// threads run two to an SM
+// threads and FP64 ones of run-time lengths two, FP32 ones of run-time lengths
+// three
 template <class C, int LGN>
 constexpr int fft_blocks() {
+  if constexpr (LGN == 0) return sizeof(C) == 16 ? 2 : 3;
   return LGN >= 8 ? 2 : 1;
 }
 
@@ -976,7 +1078,7 @@ __global__ void __launch_bounds__((fft_threads<C, LGN>()), (fft_blocks<C, LGN>()
                                      [&](int l, int x, C v) { in[T::at(l, x)] = v; });
     __syncthreads();
   } else {
-    res = fft_lines<C>(in, lc, KC >> 1, N, twx_of<C>(a), false);
+    res = fft_lines<C>(in, lc, KC >> 1, N, twx_of<C>(a), a.tmx, false);
   }
   // separate the two rows of each line; write the columns m = 0..N/2
   C* spec = reinterpret_cast<C*>(a.spec);
@@ -1039,7 +1141,7 @@ __global__ void __launch_bounds__((fft_threads<C, LGN>()), (fft_blocks<C, LGN>()
     in[il * ld + swz(jl)] = plane[(long long)jl * Nx + i0 + il];
   }
   __syncthreads();
-  const C* res = fft_lines<C>(in, ic, IC, N, twy_of<C>(a), INV);
+  const C* res = fft_lines<C>(in, ic, IC, N, twy_of<C>(a), a.tmy, INV);
   const double sc = INV ? 1.0 / (double)N : 1.0;
 #pragma unroll 4
   for (int e = threadIdx.x; e < N * IC; e += kFftThreads) {
@@ -1284,7 +1386,7 @@ __global__ void __launch_bounds__((fft_threads<C, LGN>()), (fft_blocks<C, LGN>()
     }
   }
   __syncthreads();
-  const C* res = fft_lines<C>(in, lc, KC >> 1, N, twx_of<C>(a), true);
+  const C* res = fft_lines<C>(in, lc, KC >> 1, N, twx_of<C>(a), a.tmx, true);
 #pragma unroll 4
   for (int e = threadIdx.x; e < N * KC; e += kFftThreads) {
     int kl = 0, il = 0;
@@ -1358,8 +1460,27 @@ bool fft_sizes_ok(const pb_dims* d) {
   return true;
 }
 
+// Outputs per thread of a direct transform (dft_rows): the smallest divisor
+// of N among the built ones that gives all outputs of a block's lines a
+// thread in one round, else the largest; the twiddle table (TM N values) has
+// to leave room for two blocks of 80 KiB of lines per SM (FP64) or three of
+// 48 KiB (FP32).  0: none divides N (or N is a power of two), dft_any.
+int direct_outputs(long long N, int lines, size_t elem) {
+  if (pow2(N)) return 0;
+  int best = 0;
+  const int built[] = {4, 5, 6, 8, 10};
+  for (int tm : built) {
+    if (N % tm != 0 || tm * N * (long long)elem > 24 * 1024) continue;
+    best = tm;
+    if (lines * (N / tm) <= kFftThreads) break;
+  }
+  return best;
+}
+
 size_t fft_smem(long long N, int lines, size_t elem) {
-  return (size_t)(pow2(N) ? 1 : 2) * (size_t)line_ld((int)N) * lines * elem;
+  if (pow2(N)) return (size_t)line_ld((int)N) * lines * elem;
+  const int tm = direct_outputs(N, lines, elem);  // a second set of lines and the twiddles
+  return (2 * (size_t)line_ld((int)N) * lines + (size_t)N * (tm > 0 ? tm : 1)) * elem;
 }
 
 // Lines per FFT block: a power of two, up to 16, with nlines * N <=
@@ -1501,7 +1622,7 @@ static size_t ct_smem(int lg) {
 // y-FFT and inverse x-FFT (to dst).
 struct FftShape {
   long long Nx, Ny, nz, Nh;
-  int LC, KC, IC, lgx, lgy;
+  int LC, KC, IC, lgx, lgy, tmx, tmy;
   size_t smx, smy;
   dim3 gx, gy;
 };
@@ -1519,6 +1640,8 @@ static int fft_shape(const Geo& g, FftShape& f) {
   f.smx = f.lgx ? ct_smem<C>(f.lgx) : fft_smem(f.Nx, f.LC, sizeof(C));
   f.IC = f.lgy ? ct_lines(f.lgy) : lines_for(f.Ny, sizeof(C));
   f.smy = f.lgy ? ct_smem<C>(f.lgy) : fft_smem(f.Ny, f.IC, sizeof(C));
+  f.tmx = direct_outputs(f.Nx, f.LC, sizeof(C));
+  f.tmy = direct_outputs(f.Ny, f.IC, sizeof(C));
   f.gx = dim3((unsigned)f.Ny, ceil_div(f.nz, f.KC));
   f.gy = dim3(ceil_div(f.Nh, f.IC), (unsigned)f.nz);
   return PB_OK;
@@ -1529,6 +1652,8 @@ static int fft_forward(const Geo& g, PArgs& a, int src, cudaStream_t st) {
   FftShape f;
   int rc = fft_shape<C>(g, f);
   if (rc) return rc;
+  a.tmx = f.tmx;
+  a.tmy = f.tmy;
   PB_FFT_DISPATCH(f.lgx, rc = (launch_x_fwd<C, L_>(g, a, src, f.gx, f.smx, f.KC, st)));
   if (rc) return rc;
   pb_note_launch();
@@ -1560,6 +1685,8 @@ static int fft_inverse(const Geo& g, PArgs& a, int dst, cudaStream_t st) {
   FftShape f;
   int rc = fft_shape<C>(g, f);
   if (rc) return rc;
+  a.tmx = f.tmx;
+  a.tmy = f.tmy;
   PB_FFT_DISPATCH(f.lgy, rc = (launch_y<C, L_>(g, a, true, f.gy, f.smy, f.IC, st)));
   if (rc) return rc;
   pb_note_launch();

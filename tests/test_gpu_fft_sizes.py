@@ -1,0 +1,26 @@
+"""The pressure solve on horizontal sizes that are no powers of two (products
+of the factors 2, 3, 5, 7 in every mix of the register radices, larger prime
+factors, primes) and on the short power-of-two lengths, against the FP64
+oracle: pressure 1e-11 (the plain form's tolerance) and, in the precision
+form with one refinement sweep, 1e-7 (the level means it cannot correct)."""
+import pytest
+
+from helpers import gpu_dv, gpu_sim, host_case, oracle_sim, rel_l2
+from test_gpu_precision import _stir
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(96, 90), (150, 12), (100, 21), (49, 35), (22, 26), (97, 6), (18, 54), (30, 125), (13, 81), (32, 64)]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("nx,ny", SIZES)
+def test_pressure_on_composite_lengths(nx, ny, precision):
+    nl, rs, f = host_case(case="bomex", nx=nx, ny=ny, nz=7, dx=100.0, dy=100.0, dz=40.0)
+    f = _stir(f)
+    o, g = oracle_sim(nl, rs, f), gpu_sim(nl, rs, f, precision=precision)
+    o.update_all_bcs()
+    g.PV.Update_all_bcs(g.Gr)
+    o.pr_update()
+    g.Pr.update(g.Gr, g.RS, g.DV, g.PV)
+    assert rel_l2(gpu_dv(g)["dynamic_pressure"], o.dv["dynamic_pressure"]) < (1e-11 if precision == "fp64" else 1e-7)
