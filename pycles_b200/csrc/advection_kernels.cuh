@@ -68,18 +68,87 @@ struct St {
 };
 
 namespace {
+constexpr int kMarchThreads = 128;
+
+// Whether rows of nz cells, n to a warp, leave more than 1/share of the lanes idle.
+__host__ __device__ __forceinline__ bool rows_waste(unsigned nz, unsigned n, unsigned share) {
+  const unsigned lanes = (nz + n - 1) / n * n;
+  return (lanes - nz) * share > lanes;
+}
+
+// The column (other axis o, level k) of a marching thread.  Blocks of 32
+// levels by 4 rows; where that leaves more than a tenth of the lanes idle the
+// threads run through the interior columns instead, levels fastest (a warp
+// then crosses rows and touches a sector more per access).  Measured,
+// momentum along x and y, FP64: 101 levels (21% idle) 193 and 182 us by rows,
+// 150 and 162 flat, at 200x180; 150 levels (6%) 67 and 56 us by rows, 74 and
+// 60 flat, at 96x96.
+__device__ __forceinline__ bool march_column(const Geo& g, long long n_other, long long& o, long long& k) {
+  const unsigned nz = (unsigned)(g.n2 - 2 * g.gw), no = (unsigned)(n_other - 2 * g.gw);
+  unsigned q, r;
+  if (rows_waste(nz, 32, 10)) {
+    const unsigned p = blockIdx.x * kMarchThreads + threadIdx.x;
+    q = p / nz;
+    r = p - q * nz;
+  } else {
+    q = blockIdx.y * 4 + (threadIdx.x >> 5);
+    r = blockIdx.x * 32 + (threadIdx.x & 31);
+  }
+  o = g.gw + q;
+  k = g.gw + r;
+  return q < no && r < nz;
+}
+inline dim3 march_grid(long long n_other, long long nz, long long chunks) {
+  return rows_waste((unsigned)nz, 32, 10) ? dim3(ceil_div(n_other * nz, kMarchThreads), 1, (unsigned)chunks)
+                                          : dim3(ceil_div(nz, 32), ceil_div(n_other, 4), (unsigned)chunks);
+}
+inline long long march_blocks(long long n_other, long long nz) {
+  const dim3 b = march_grid(n_other, nz, 1);
+  return (long long)b.x * b.y;
+}
+
+// The row j and face f (the face above cell f) of a lane of the z kernels.  A
+// warp takes 32 consecutive faces, the first only for the face below the
+// second's cell; every later lane owns the cell below its face.  By rows: 31
+// cells of a row to a warp; where that leaves more than 1/16 of the lanes
+// idle, 32 consecutive ones of the (nz + 1) faces of the rows of an x plane
+// (a row's lowest face owns no cell).  Measured, scalars, FP64: 128 levels
+// (17% idle) 220 us by rows, 187 flat, at 256x256; 150 levels (3%) 42 and 45
+// at 96x96; FP32, 256 levels (8%) 667 and 638 at 512x512.
+__device__ __forceinline__ bool z_face(const Geo& g, int lane, long long& j, long long& f, bool& cell) {
+  const unsigned nz = (unsigned)(g.n2 - 2 * g.gw), nj = (unsigned)(g.n1 - 2 * g.gw);
+  const unsigned w = threadIdx.x >> 5;
+  unsigned q, r;
+  if (rows_waste(nz, 31, 16)) {
+    const unsigned t = (blockIdx.x * (kMarchThreads / 32) + w) * 31 + lane;
+    q = t / (nz + 1);
+    r = t - q * (nz + 1);
+  } else {
+    q = blockIdx.y * (kMarchThreads / 32) + w;
+    r = blockIdx.x * 31 + lane;
+  }
+  j = g.gw + q;
+  f = g.gw - 1 + r;
+  const bool valid = q < nj && r <= nz;
+  cell = valid && lane > 0 && r > 0;
+  return valid;
+}
+inline dim3 z_grid(long long nl0, long long nl1, long long nl2) {
+  constexpr int W = kMarchThreads / 32;
+  return rows_waste((unsigned)nl2, 31, 16) ? dim3(ceil_div(nl1 * (nl2 + 1), 31 * W), 1, (unsigned)nl0)
+                                           : dim3(ceil_div(nl2, 31), ceil_div(nl1, W), (unsigned)nl0);
+}
+
 // ---------------------------------------------------------------------------
 // scalars, x / y directions
 // ---------------------------------------------------------------------------
 template <int D, int ORDER, bool F32, int NS>
-__global__ void __launch_bounds__(128) scalar_march(Geo g, ScalarArgs a, int chunk) {
+__global__ void __launch_bounds__(kMarchThreads) scalar_march(Geo g, ScalarArgs a, int chunk) {
   constexpr int R = St<ORDER>::R;
   constexpr int W = St<ORDER>::W;
-  const long long k = g.gw + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long o = g.gw + (long long)blockIdx.y * blockDim.y + threadIdx.y;
   const long long nD = (D == 0) ? g.n0 : g.n1;
-  const long long nO = (D == 0) ? g.n1 : g.n0;
-  if (k >= g.n2 - g.gw || o >= nO - g.gw) return;
+  long long o, k;
+  if (!march_column(g, (D == 0) ? g.n1 : g.n0, o, k)) return;
   const long long sD = (D == 0) ? g.is : g.js;
   const long long sO = (D == 0) ? g.js : g.is;
   const long long c0 = g.gw + (long long)blockIdx.z * chunk;
@@ -126,16 +195,13 @@ __global__ void __launch_bounds__(128) scalar_march(Geo g, ScalarArgs a, int chu
 // scalars, z direction
 // ---------------------------------------------------------------------------
 template <int ORDER, bool F32, int NS>
-__global__ void __launch_bounds__(128) scalar_z(Geo g, ScalarArgs a) {
+__global__ void __launch_bounds__(kMarchThreads) scalar_z(Geo g, ScalarArgs a) {
   constexpr int R = St<ORDER>::R;
   const int lane = threadIdx.x & 31;
-  // grid (segment, group of 4 rows, x): warp w of the block takes row 4*blockIdx.y + w
-  const long long seg = blockIdx.x;
-  const long long j = g.gw + (long long)blockIdx.y * 4 + (threadIdx.x >> 5);
+  long long j, f;
+  bool cell;
+  const bool valid = z_face(g, lane, j, f, cell);
   const long long i = g.gw + (long long)blockIdx.z;
-  if (j >= g.n1 - g.gw) return;  // whole warps
-  const long long f = g.gw + seg * 31 - 1 + lane;   // face of this lane = cell of this lane
-  const bool valid = f <= g.n2 - g.gw - 1;
   const long long col = i * g.is + j * g.js;
   const double dzi = g.dxi2;
 #pragma unroll
@@ -151,7 +217,7 @@ __global__ void __launch_bounds__(128) scalar_z(Geo g, ScalarArgs a) {
       if (a.flux[q] != nullptr) a.flux[q][col + f] = F;
     }
     const double Fm = __shfl_up_sync(0xffffffffu, F, 1);
-    if (valid && lane > 0) a.t[q][col + f] -= a.alpha0_half[f] * (F - Fm) * dzi;
+    if (cell) a.t[q][col + f] -= a.alpha0_half[f] * (F - Fm) * dzi;
   }
 }
 
@@ -167,14 +233,12 @@ __global__ void __launch_bounds__(128) scalar_z(Geo g, ScalarArgs a) {
 // stepping), so it stores the x term instead of adding it to the stored
 // value (0 - x, as the reference's accumulation into a zeroed tendency).
 template <int D, int ORDER, bool SET>
-__global__ void __launch_bounds__(128) scalar_march_f32(Geo g, ScalarArgs a, int chunk) {
+__global__ void __launch_bounds__(kMarchThreads) scalar_march_f32(Geo g, ScalarArgs a, int chunk) {
   constexpr int R = St<ORDER>::R;
   constexpr int ND = 2 * R - 1;
-  const long long k = g.gw + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long o = g.gw + (long long)blockIdx.y * blockDim.y + threadIdx.y;
   const long long nD = (D == 0) ? g.n0 : g.n1;
-  const long long nO = (D == 0) ? g.n1 : g.n0;
-  if (k >= g.n2 - g.gw || o >= nO - g.gw) return;
+  long long o, k;
+  if (!march_column(g, (D == 0) ? g.n1 : g.n0, o, k)) return;
   const long long sD = (D == 0) ? g.is : g.js;
   const long long sO = (D == 0) ? g.js : g.is;
   const long long c0 = g.gw + (long long)blockIdx.z * chunk;
@@ -238,17 +302,14 @@ __global__ void __launch_bounds__(128) scalar_march_f32(Geo g, ScalarArgs a, int
 // warps still read the current values) and, at stage 0, the copy; the
 // tendency is not stored.
 template <int ORDER, bool RK>
-__global__ void __launch_bounds__(128) scalar_z_f32(Geo g, ScalarArgs a) {
+__global__ void __launch_bounds__(kMarchThreads) scalar_z_f32(Geo g, ScalarArgs a) {
   constexpr int R = St<ORDER>::R;
   constexpr int ND = 2 * R - 1;
   const int lane = threadIdx.x & 31;
-  // grid (segment, group of 4 rows, x): warp w of the block takes row 4*blockIdx.y + w
-  const long long seg = blockIdx.x;
-  const long long j = g.gw + (long long)blockIdx.y * 4 + (threadIdx.x >> 5);
+  long long j, f;
+  bool cell;
+  const bool valid = z_face(g, lane, j, f, cell);
   const long long i = g.gw + (long long)blockIdx.z;
-  if (j >= g.n1 - g.gw) return;  // whole warps
-  const long long f = g.gw + seg * 31 - 1 + lane;
-  const bool valid = f <= g.n2 - g.gw - 1;
   const long long col = i * g.is + j * g.js;
   double F = 0.0, val = 0.0;
   if (valid) {
@@ -266,7 +327,7 @@ __global__ void __launch_bounds__(128) scalar_z_f32(Geo g, ScalarArgs a) {
     val = w[R - 1];
   }
   const double Fm = __shfl_up_sync(0xffffffffu, F, 1);
-  if (valid && lane > 0) {
+  if (cell) {
     const long long at = col + f;
     const double t = fma(-a.alpha0_half[f] * g.dxi2, F - Fm, a.t[0][at]);
     if constexpr (RK) {
@@ -290,15 +351,13 @@ __global__ void __launch_bounds__(128) scalar_z_f32(Geo g, ScalarArgs a) {
 // momentum, x / y directions (advecting velocity = component D)
 // ---------------------------------------------------------------------------
 template <int D, int ORDER, bool F32>
-__global__ void __launch_bounds__(128) momentum_march(Geo g, MomArgs a, int chunk) {
+__global__ void __launch_bounds__(kMarchThreads) momentum_march(Geo g, MomArgs a, int chunk) {
   constexpr int R = St<ORDER>::R;
   constexpr int W = St<ORDER>::W;
   constexpr int O = 1 - D;  // other horizontal axis
-  const long long k = g.gw + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long o = g.gw + (long long)blockIdx.y * blockDim.y + threadIdx.y;
   const long long nD = (D == 0) ? g.n0 : g.n1;
-  const long long nO = (D == 0) ? g.n1 : g.n0;
-  if (k >= g.n2 - g.gw || o >= nO - g.gw) return;
+  long long o, k;
+  if (!march_column(g, (D == 0) ? g.n1 : g.n0, o, k)) return;
   const long long sD = (D == 0) ? g.is : g.js;
   const long long sO = (D == 0) ? g.js : g.is;
   const long long c0 = g.gw + (long long)blockIdx.z * chunk;
@@ -368,15 +427,12 @@ __global__ void __launch_bounds__(128) momentum_march(Geo g, MomArgs a, int chun
 // momentum, z direction (advecting velocity = w)
 // ---------------------------------------------------------------------------
 template <int ORDER, bool F32>
-__global__ void __launch_bounds__(128) momentum_z(Geo g, MomArgs a) {
+__global__ void __launch_bounds__(kMarchThreads) momentum_z(Geo g, MomArgs a) {
   const int lane = threadIdx.x & 31;
-  // grid (segment, group of 4 rows, x): warp w of the block takes row 4*blockIdx.y + w
-  const long long seg = blockIdx.x;
-  const long long j = g.gw + (long long)blockIdx.y * 4 + (threadIdx.x >> 5);
+  long long j, f;
+  bool cell;
+  const bool valid = z_face(g, lane, j, f, cell);
   const long long i = g.gw + (long long)blockIdx.z;
-  if (j >= g.n1 - g.gw) return;  // whole warps
-  const long long f = g.gw + seg * 31 - 1 + lane;
-  const bool valid = f <= g.n2 - g.gw - 1;
   const long long idx = i * g.is + j * g.js + f;
   const double dzi = g.dxi2;
   const double* wv = a.vel[2];
@@ -400,7 +456,7 @@ __global__ void __launch_bounds__(128) momentum_z(Geo g, MomArgs a) {
       F = upwind_flux1(vel_adv, weno_upwind<ORDER, F32>(vel_adv >= 0.0, v), rho);
     }
     const double Fm = __shfl_up_sync(0xffffffffu, F, 1);
-    if (valid && lane > 0) {
+    if (cell) {
       const double al = (c == 2) ? a.alpha0[f] : a.alpha0_half[f];
       a.tend[c][idx] -= al * (F - Fm) * dzi;
     }
@@ -677,21 +733,28 @@ constexpr int kChunk = 64;  // cells per marching thread along x / y, at most (m
 
 // Cells per block along the marching direction.  The grid runs in waves of
 // sms x per_sm resident blocks and a block takes ~chunk + lead steps (lead:
-// its window fill), so the chunk in [8, max_chunk] with the fewest
+// its window fill), so the chunk in [min_chunk, max_chunk] with the fewest
 // wave-steps is taken (ties: the longer chunk).  A fixed 64 left the last
 // wave nearly empty at 512x512x256 (2520 blocks of the momentum pass on 148
 // SMs: 17.03 waves) and most SMs idle on small grids (15 blocks at
+// 64x64x75).  A thread's steps are a chain of one face after another; on a
+// grid of one wave the chain's length is the kernel's time, and the window
+// fill, loads without that chain, counts about `fill` steps: the
+// marching kernels take chunks down to one cell there (momentum, x, FP64:
+// 6.6 us at 32x32x32, 21.7 with chunks of 8; 19.6 against 25.7 at
 // 64x64x75).  The results do not depend on the chunk: a face on a chunk
 // boundary is evaluated by both blocks with the same arithmetic.
-inline int march_chunk(long long n_march, long long other_blocks, int per_sm, int lead, int max_chunk) {
+inline int march_chunk(long long n_march, long long other_blocks, int per_sm, int lead, int max_chunk,
+                       int min_chunk = 8, int fill = -1) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long slots = (long long)sms * (per_sm > 0 ? per_sm : 1);
   int best = max_chunk;
   long long best_cost = -1;
-  for (int c = 8; c <= max_chunk; ++c) {
+  for (int c = min_chunk; c <= max_chunk; ++c) {
     const long long blocks = other_blocks * ((n_march + c - 1) / c);
-    const long long cost = (blocks + slots - 1) / slots * (c + lead);
+    const long long waves = (blocks + slots - 1) / slots;
+    const long long cost = (waves - 1) * (c + lead) + c + (fill >= 0 ? fill : lead);
     if (best_cost < 0 || cost <= best_cost) {
       best_cost = cost;
       best = c;
@@ -712,25 +775,24 @@ cudaError_t launch_scalar_group(const Geo& g, ScalarArgs base, double* const* fl
                                 const double* const vel[3], cudaStream_t st) {
   constexpr int R = St<ORDER>::R;
   const long long nl0 = g.n0 - 2 * g.gw, nl1 = g.n1 - 2 * g.gw, nl2 = g.n2 - 2 * g.gw;
-  dim3 blk(32, 4);
   {
     ScalarArgs a = base;
     a.vel = vel[0];
     for (int q = 0; q < NS; ++q) a.flux[q] = flux_dir[0] ? flux_dir[0][q] : nullptr;
-    const long long other = (long long)ceil_div(nl2, 32) * ceil_div(nl1, 4);
+    const long long other = march_blocks(nl1, nl2);
     if constexpr (F32 && NS == 1) {
       if (a.fused) {
-        const int c = march_chunk(nl0, other, resident_blocks(scalar_march_f32<0, ORDER, true>, 128), 2 * R, kChunk);
-        scalar_march_f32<0, ORDER, true><<<dim3(ceil_div(nl2, 32), ceil_div(nl1, 4), ceil_div(nl0, c)), blk, 0, st>>>(
+        const int c = march_chunk(nl0, other, resident_blocks(scalar_march_f32<0, ORDER, true>, 128), 2 * R, kChunk, 1, 2);
+        scalar_march_f32<0, ORDER, true><<<march_grid(nl1, nl2, ceil_div(nl0, c)), kMarchThreads, 0, st>>>(
             g, a, c);
       } else {
-        const int c = march_chunk(nl0, other, resident_blocks(scalar_march_f32<0, ORDER, false>, 128), 2 * R, kChunk);
-        scalar_march_f32<0, ORDER, false><<<dim3(ceil_div(nl2, 32), ceil_div(nl1, 4), ceil_div(nl0, c)), blk, 0, st>>>(
+        const int c = march_chunk(nl0, other, resident_blocks(scalar_march_f32<0, ORDER, false>, 128), 2 * R, kChunk, 1, 2);
+        scalar_march_f32<0, ORDER, false><<<march_grid(nl1, nl2, ceil_div(nl0, c)), kMarchThreads, 0, st>>>(
             g, a, c);
       }
     } else {
-      const int c = march_chunk(nl0, other, resident_blocks(scalar_march<0, ORDER, F32, NS>, 128), 2 * R, kChunk);
-      scalar_march<0, ORDER, F32, NS><<<dim3(ceil_div(nl2, 32), ceil_div(nl1, 4), ceil_div(nl0, c)), blk, 0, st>>>(
+      const int c = march_chunk(nl0, other, resident_blocks(scalar_march<0, ORDER, F32, NS>, 128), 2 * R, kChunk, 1, 2);
+      scalar_march<0, ORDER, F32, NS><<<march_grid(nl1, nl2, ceil_div(nl0, c)), kMarchThreads, 0, st>>>(
           g, a, c);
     }
     pb_note_launch();
@@ -739,14 +801,14 @@ cudaError_t launch_scalar_group(const Geo& g, ScalarArgs base, double* const* fl
     ScalarArgs a = base;
     a.vel = vel[1];
     for (int q = 0; q < NS; ++q) a.flux[q] = flux_dir[1] ? flux_dir[1][q] : nullptr;
-    const long long other = (long long)ceil_div(nl2, 32) * ceil_div(nl0, 4);
+    const long long other = march_blocks(nl0, nl2);
     if constexpr (F32 && NS == 1) {
-      const int c = march_chunk(nl1, other, resident_blocks(scalar_march_f32<1, ORDER, false>, 128), 2 * R, kChunk);
-      scalar_march_f32<1, ORDER, false><<<dim3(ceil_div(nl2, 32), ceil_div(nl0, 4), ceil_div(nl1, c)), blk, 0, st>>>(
+      const int c = march_chunk(nl1, other, resident_blocks(scalar_march_f32<1, ORDER, false>, 128), 2 * R, kChunk, 1, 2);
+      scalar_march_f32<1, ORDER, false><<<march_grid(nl0, nl2, ceil_div(nl1, c)), kMarchThreads, 0, st>>>(
           g, a, c);
     } else {
-      const int c = march_chunk(nl1, other, resident_blocks(scalar_march<1, ORDER, F32, NS>, 128), 2 * R, kChunk);
-      scalar_march<1, ORDER, F32, NS><<<dim3(ceil_div(nl2, 32), ceil_div(nl0, 4), ceil_div(nl1, c)), blk, 0, st>>>(
+      const int c = march_chunk(nl1, other, resident_blocks(scalar_march<1, ORDER, F32, NS>, 128), 2 * R, kChunk, 1, 2);
+      scalar_march<1, ORDER, F32, NS><<<march_grid(nl0, nl2, ceil_div(nl1, c)), kMarchThreads, 0, st>>>(
           g, a, c);
     }
     pb_note_launch();
@@ -755,14 +817,14 @@ cudaError_t launch_scalar_group(const Geo& g, ScalarArgs base, double* const* fl
     ScalarArgs a = base;
     a.vel = vel[2];
     for (int q = 0; q < NS; ++q) a.flux[q] = flux_dir[2] ? flux_dir[2][q] : nullptr;
-    const dim3 grd(ceil_div(nl2, 31), ceil_div(nl1, 4), (unsigned)nl0);
+    const dim3 grd = z_grid(nl0, nl1, nl2);
     if constexpr (F32 && NS == 1) {
       if (a.fused)
-        scalar_z_f32<ORDER, true><<<grd, 128, 0, st>>>(g, a);
+        scalar_z_f32<ORDER, true><<<grd, kMarchThreads, 0, st>>>(g, a);
       else
-        scalar_z_f32<ORDER, false><<<grd, 128, 0, st>>>(g, a);
+        scalar_z_f32<ORDER, false><<<grd, kMarchThreads, 0, st>>>(g, a);
     } else {
-      scalar_z<ORDER, F32, NS><<<grd, 128, 0, st>>>(g, a);
+      scalar_z<ORDER, F32, NS><<<grd, kMarchThreads, 0, st>>>(g, a);
     }
     pb_note_launch();
   }
@@ -806,7 +868,6 @@ cudaError_t launch_scalar_ns(int ns, const Geo& g, ScalarArgs base, double* cons
 template <int ORDER, bool F32>
 cudaError_t launch_momentum(const Geo& g, const MomArgs& a, cudaStream_t st) {
   const long long nl0 = g.n0 - 2 * g.gw, nl1 = g.n1 - 2 * g.gw, nl2 = g.n2 - 2 * g.gw;
-  dim3 blk(32, 4);
   constexpr int R = St<ORDER>::R;
   if constexpr (F32) {  // precision form: one pass for the three advecting directions
     using T = MomTile<ORDER>;
@@ -816,17 +877,15 @@ cudaError_t launch_momentum(const Geo& g, const MomArgs& a, cudaStream_t st) {
     pb_note_launch();
     return cudaGetLastError();
   } else {
-  const int c0 = march_chunk(nl0, (long long)ceil_div(nl2, 32) * ceil_div(nl1, 4),
-                             resident_blocks(momentum_march<0, ORDER, F32>, 128), 2 * R, kChunk);
-  momentum_march<0, ORDER, F32><<<dim3(ceil_div(nl2, 32), ceil_div(nl1, 4), ceil_div(nl0, c0)), blk, 0,
-                                  st>>>(g, a, c0);
+  const int c0 = march_chunk(nl0, march_blocks(nl1, nl2),
+                             resident_blocks(momentum_march<0, ORDER, F32>, 128), 2 * R, kChunk, 1, 2);
+  momentum_march<0, ORDER, F32><<<march_grid(nl1, nl2, ceil_div(nl0, c0)), kMarchThreads, 0, st>>>(g, a, c0);
   pb_note_launch();
-  const int c1 = march_chunk(nl1, (long long)ceil_div(nl2, 32) * ceil_div(nl0, 4),
-                             resident_blocks(momentum_march<1, ORDER, F32>, 128), 2 * R, kChunk);
-  momentum_march<1, ORDER, F32><<<dim3(ceil_div(nl2, 32), ceil_div(nl0, 4), ceil_div(nl1, c1)), blk, 0,
-                                  st>>>(g, a, c1);
+  const int c1 = march_chunk(nl1, march_blocks(nl0, nl2),
+                             resident_blocks(momentum_march<1, ORDER, F32>, 128), 2 * R, kChunk, 1, 2);
+  momentum_march<1, ORDER, F32><<<march_grid(nl0, nl2, ceil_div(nl1, c1)), kMarchThreads, 0, st>>>(g, a, c1);
   pb_note_launch();
-  momentum_z<ORDER, F32><<<dim3(ceil_div(nl2, 31), ceil_div(nl1, 4), (unsigned)nl0), 128, 0, st>>>(g, a);
+  momentum_z<ORDER, F32><<<z_grid(nl0, nl1, nl2), kMarchThreads, 0, st>>>(g, a);
   pb_note_launch();
   return cudaGetLastError();
   }
