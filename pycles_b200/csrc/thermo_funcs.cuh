@@ -34,20 +34,31 @@ __device__ __forceinline__ double qv_star_c(double p0, double qt, double pv) {
 }
 // alpha and buoyancy: buoyancy cancels ~3 digits of alpha, so both keep the
 // reference's separately rounded operations in either form.
-__device__ __forceinline__ double alpha_c(double p0, double T, double qt, double qv) {
-  return mul_rn((Rd * T) / p0, add_rn(sub_rn(1.0, qt), mul_rn(eps_vi, qv)));
+// Their divisors are a level's: ip0 = 1 / p0, ia0 = 1 / alpha0 (div_by).  fin:
+// T is finite; else the results are T's infinity or NaN, as a division's.
+__device__ __forceinline__ double alpha_c(double p0, double ip0, double T, double qt, double qv, bool fin) {
+  const double a = div_by(Rd * T, p0, ip0);
+  return mul_rn(fin ? a : T, add_rn(sub_rn(1.0, qt), mul_rn(eps_vi, qv)));
 }
-__device__ __forceinline__ double buoyancy_c(double alpha0, double alpha) {
-  return mul_rn(g, sub_rn(alpha, alpha0)) / alpha0;
+__device__ __forceinline__ double buoyancy_c(double alpha0, double ia0, double alpha, bool fin) {
+  const double b = div_by(mul_rn(g, sub_rn(alpha, alpha0)), alpha0, ia0);
+  return fin ? b : alpha;
 }
 __device__ __forceinline__ double cpm_c(double qt) { return (1.0 - qt) * cpd + qt * cpv; }
+// log(x / p_tilde) and log(T / T_tilde): the plain form's quotients are the
+// correctly rounded ones, formed with the constants' reciprocals (div_by); the
+// precision form multiplies by them.
 template <class M>
-__device__ __forceinline__ double sd_c(double pd, double T) {
-  return sd_tilde + cpd * M::log(T / T_tilde) - Rd * M::log(pd / p_tilde);
+__device__ __forceinline__ double log_p(double p) {
+  constexpr double y = 1.0 / p_tilde;
+  if constexpr (M::exact) return M::log(div_by(p, p_tilde, y));
+  else return M::log(p * y);
 }
 template <class M>
-__device__ __forceinline__ double sv_c(double pv, double T) {
-  return sv_tilde + cpv * M::log(T / T_tilde) - Rv * M::log(pv / p_tilde);
+__device__ __forceinline__ double log_T(double T) {
+  constexpr double y = 1.0 / T_tilde;
+  if constexpr (M::exact) return M::log(div_by(T, T_tilde, y));
+  else return M::log(T * y);
 }
 __device__ __forceinline__ double sc_c(double L, double T) { return -L / T; }
 __device__ __forceinline__ double interp_2(double a, double b) { return 0.5 * (a + b); }
@@ -75,39 +86,22 @@ __device__ __forceinline__ double table_lookup(const pb_table& t, double x, unsi
   return y1 + (x - x1) * (y2 - y1) * t.dxi;
 }
 
-// temperature_no_ql (Csrc/thermodynamics_sa.h:10-15).  The precision form
-// multiplies by 1/p_tilde instead of dividing (FP64 division is a
-// multi-instruction sequence).
+// temperature_no_ql (Csrc/thermodynamics_sa.h:10-15).
 template <class M>
 __device__ __forceinline__ double temperature_no_ql(double pd, double pv, double s, double qt) {
-  if constexpr (M::exact) {
-    return T_tilde * M::exp((s - (1.0 - qt) * (sd_tilde - Rd * M::log(pd / p_tilde)) -
-                             qt * (sv_tilde - Rv * M::log(pv / p_tilde))) /
-                            ((1.0 - qt) * cpd + qt * cpv));
-  } else {
-    constexpr double ipt = 1.0 / p_tilde;
-    return T_tilde * M::exp((s - (1.0 - qt) * (sd_tilde - Rd * M::log(pd * ipt)) -
-                             qt * (sv_tilde - Rv * M::log(pv * ipt))) /
-                            ((1.0 - qt) * cpd + qt * cpv));
-  }
+  return T_tilde * M::exp((s - (1.0 - qt) * (sd_tilde - Rd * log_p<M>(pd)) - qt * (sv_tilde - Rv * log_p<M>(pv))) /
+                          ((1.0 - qt) * cpd + qt * cpv));
 }
 
 // Entropy of the saturated mixture at temperature T (the secant's s_1, s_2,
-// Csrc/thermodynamics_sa.h:37,54): the reference's operations in the plain
-// form; the precision form evaluates log(T/T_tilde) once for the dry and the
-// vapour parts and multiplies by the constant reciprocals (three logarithms
-// per secant iteration instead of four).
+// Csrc/thermodynamics_sa.h:37,54), sd_c and sv_c (Csrc/entropies.h) with
+// log(T / T_tilde) evaluated once for both.
 template <class M>
 __device__ __forceinline__ double entropy_sat(double pd, double pv, double T, double qt, double L, double sigma) {
-  if constexpr (M::exact) {
-    return sd_c<M>(pd, T) * (1.0 - qt) + sv_c<M>(pv, T) * qt + sc_c(L, T) * sigma;
-  } else {
-    constexpr double ipt = 1.0 / p_tilde, iTt = 1.0 / T_tilde;
-    const double lT = M::log(T * iTt);
-    const double sd = sd_tilde + cpd * lT - Rd * M::log(pd * ipt);
-    const double sv = sv_tilde + cpv * lT - Rv * M::log(pv * ipt);
-    return sd * (1.0 - qt) + sv * qt + sc_c(L, T) * sigma;
-  }
+  const double lT = log_T<M>(T);
+  const double sd = sd_tilde + cpd * lT - Rd * log_p<M>(pd);
+  const double sv = sv_tilde + cpv * lT - Rv * log_p<M>(pv);
+  return sd * (1.0 - qt) + sv * qt + sc_c(L, T) * sigma;
 }
 
 // The secant's first point (Csrc/thermodynamics_sa.h:22-24): the temperature

@@ -100,18 +100,17 @@ __global__ void __launch_bounds__(kSaThreads, 4) thermo_sa_kernel(Geo geo, SaArg
   extern __shared__ __align__(16) unsigned char smraw[];
   const int lane = threadIdx.x & 31;
   const long long n2 = geo.n2;
-  // per level: the Exner function, and for the precision form the
-  // reciprocals of p0, alpha0 and the Exner function (FP64 divisions by
-  // them become multiplications)
-  double* exner_tab = reinterpret_cast<double*>(smraw);  // [n2] (x4 in the precision form)
+  // per level: the Exner function and the reciprocals of the Exner function,
+  // p0 and alpha0: the divisions by them become multiplications in the
+  // precision form and five multiply-adds (div_by, the same quotients) in the
+  // plain form
+  double* exner_tab = reinterpret_cast<double*>(smraw);  // [4][n2]
   for (int k = threadIdx.x; k < n2; k += blockDim.x) {
     const double ex = pow(a.p0[k] / p_tilde, kappa);
     exner_tab[k] = ex;
-    if constexpr (!M::exact) {
-      exner_tab[n2 + k] = 1.0 / ex;
-      exner_tab[2 * n2 + k] = 1.0 / a.p0[k];
-      exner_tab[3 * n2 + k] = 1.0 / a.alpha0[k];
-    }
+    exner_tab[n2 + k] = 1.0 / ex;
+    exner_tab[2 * n2 + k] = 1.0 / a.p0[k];
+    exner_tab[3 * n2 + k] = 1.0 / a.alpha0[k];
   }
   __syncthreads();
   const long long ntask = ncols * nseg;
@@ -154,19 +153,23 @@ __global__ void __launch_bounds__(kSaThreads, 4) thermo_sa_kernel(Geo geo, SaArg
       T = e.T;
       qv = e.qv;
       double al;
+      const bool fin = isfinite(T);
       if constexpr (M::exact) {
-        al = alpha_c(p0, T, qt, qv);
+        al = alpha_c(p0, exner_tab[2 * n2 + k], T, qt, qv, fin);
         // bvf_sa first loop (:147-157): theta_rho on k in [1, n2-1)
-        if (k >= 1 && k < n2 - 1) thr = T * (1.0 - qt + eps_vi * qv) / exner;
+        if (k >= 1 && k < n2 - 1) {
+          const double t = T * (1.0 - qt + eps_vi * qv);
+          thr = fin ? div_by(t, exner, exner_tab[n2 + k]) : t;
+        }
         // buoyancy_update_sa first loop (:110-119): k in [0, n2-1)
-        if (k < n2 - 1) b = buoyancy_c(a0, al);
+        if (k < n2 - 1) b = buoyancy_c(a0, exner_tab[3 * n2 + k], al, fin);
       } else {
         al = (Rd * T) * exner_tab[2 * n2 + k] * (1.0 - qt + eps_vi * qv);
         if (k >= 1 && k < n2 - 1) thr = T * (1.0 - qt + eps_vi * qv) * exner_tab[n2 + k];
         if (k < n2 - 1) b = g * (al - a0) * exner_tab[3 * n2 + k];
       }
       if (own) {
-        if (!isfinite(T)) pb_flag_at(a.err, PB_ERR_NONFINITE);
+        if (!fin) pb_flag_at(a.err, PB_ERR_NONFINITE);
         my_it += (unsigned long long)e.iters;
         my_sat += e.sat ? 1ull : 0ull;
         a.T[idx] = T;
@@ -176,7 +179,8 @@ __global__ void __launch_bounds__(kSaThreads, 4) thermo_sa_kernel(Geo geo, SaArg
         a.alpha[idx] = al;
         // thetali_update (:185-211) with thetali_c (thermodynamic_functions.h:15-18);
         // without condensate the exponential is exp(-0) = 1 exactly
-        const double theta = M::exact ? T / exner : T * exner_tab[n2 + k];
+        const double theta =
+            M::exact ? (fin ? div_by(T, exner, exner_tab[n2 + k]) : T) : T * exner_tab[n2 + k];
         if (e.ql == 0.0 && e.qi == 0.0) {
           a.thetali[idx] = theta * 1.0;
         } else {
@@ -227,61 +231,70 @@ __global__ void __launch_bounds__(kSaThreads, 4) thermo_sa_kernel(Geo geo, SaArg
   }
 }
 
-// ThermodynamicsDry.update (ThermodynamicsDry.pyx:105-120).
+// ThermodynamicsDry.update (ThermodynamicsDry.pyx:105-120).  A thread keeps
+// one level: what depends on the level alone (log(p0 / p_tilde), the Exner
+// function, the divisors' reciprocals) is formed once and the block walks over
+// columns, resident blocks only.  One column per block evaluated the level's
+// log and pow for every cell: 266 us at 256x256x128 (FP64), 223 now.
 template <class M>
-__global__ void thermo_dry_kernel(Geo geo, DryArgs a, long long ncols) {
+__global__ void __launch_bounds__(1024) thermo_dry_kernel(Geo geo, DryArgs a, long long ncols) {
   extern __shared__ __align__(16) unsigned char smraw[];
   double* sm = reinterpret_cast<double*>(smraw);
   const int kpad = blockDim.x;
-  const long long col = (long long)blockIdx.x * blockDim.y + threadIdx.y;
   const int k = threadIdx.x;
   const long long n2 = geo.n2;
   double* sTh = sm + (size_t)threadIdx.y * 2 * kpad;
   double* sB = sTh + kpad;
-  const bool active = (col < ncols) && (k < n2);
-  const long long i = col / geo.n1;
-  const long long j = col - i * geo.n1;
-  long long idx = 0;
-  double T = 0.0;
-  if (active) {
-    idx = col * n2 + k;
-    const double pd = a.pd[k];
-    // eos_c (Csrc/thermodynamics_dry.h:8-10), eos_update (:12-37)
-    T = T_tilde * (M::exp((a.s[idx] - sd_tilde + Rd * M::log(pd / p_tilde)) / cpd));
-    a.T[idx] = T;
-    const double al = mul_rn((Rd * T) / pd, 1.0);
-    a.alpha[idx] = al;
-    // buoyancy_update (:39-73): i < n0-1, j < n1-1, k < n2-1
+  const bool kin = k < n2;
+  const double pd = kin ? a.pd[k] : 1.0, a0 = kin ? a.alpha0[k] : 1.0;
+  const double lp = M::log(pd / p_tilde), ex = pow(pd / p_tilde, kappa);
+  const double ipd = 1.0 / pd, ia0 = 1.0 / a0, iex = 1.0 / ex;
+  const double dzi = 1.0 / geo.dx2;
+  for (long long c0 = (long long)blockIdx.x * blockDim.y; c0 < ncols; c0 += (long long)gridDim.x * blockDim.y) {
+    const long long col = c0 + threadIdx.y;
+    const bool active = col < ncols && kin;
+    const long long i = col / geo.n1;
+    const long long j = col - i * geo.n1;
+    const long long idx = col * n2 + k;
     const bool bij = (i < geo.n0 - 1) && (j < geo.n1 - 1);
-    double b = 0.0;
-    if (bij && k < n2 - 1) {
-      b = buoyancy_c(a.alpha0[k], al);
-      a.buoy[idx] = b;
-    } else if (bij) {
-      b = a.buoy[idx];  // level n2-1 keeps the field's current value
+    if (active) {
+      // eos_c (Csrc/thermodynamics_dry.h:8-10), eos_update (:12-37)
+      constexpr double icp = 1.0 / cpd;
+      const double T = T_tilde * (M::exp(div_by(a.s[idx] - sd_tilde + Rd * lp, cpd, icp)));
+      const bool fin = isfinite(T);
+      a.T[idx] = T;
+      const double al = mul_rn(fin ? div_by(Rd * T, pd, ipd) : T, 1.0);
+      a.alpha[idx] = al;
+      // buoyancy_update (:39-73): i < n0-1, j < n1-1, k < n2-1
+      double b = 0.0;
+      if (bij && k < n2 - 1) {
+        b = buoyancy_c(a0, ia0, al, fin);
+        a.buoy[idx] = b;
+      } else if (bij) {
+        b = a.buoy[idx];  // level n2-1 keeps the field's current value
+      }
+      sB[k] = b;
+      // bvf_dry (:75-110): theta on k in [1, n2)
+      double th = 0.0;
+      if (k >= 1) {
+        th = fin ? div_by(T, ex, iex) : T;
+        a.theta[idx] = th;
+      }
+      sTh[k] = th;
     }
-    sB[k] = b;
-    // bvf_dry (:75-110): theta on k in [1, n2)
-    double th = 0.0;
-    if (k >= 1) {
-      th = T / pow(pd / p_tilde, kappa);
-      a.theta[idx] = th;
+    __syncthreads();
+    if (active) {
+      if (bij && k < n2 - 1) a.wt[idx] += interp_2(sB[k], sB[k + 1]);
+      if (k >= 2 && k < n2 - 1)
+        a.bvf[idx] = g / sTh[k] * (interp_2(sTh[k], sTh[k + 1]) - interp_2(sTh[k - 1], sTh[k])) * dzi;
     }
-    sTh[k] = th;
-  }
-  __syncthreads();
-  if (active) {
-    if ((i < geo.n0 - 1) && (j < geo.n1 - 1) && k < n2 - 1) a.wt[idx] += interp_2(sB[k], sB[k + 1]);
-    if (k >= 2 && k < n2 - 1) {
-      const double dzi = 1.0 / geo.dx2;
-      a.bvf[idx] = g / sTh[k] * (interp_2(sTh[k], sTh[k + 1]) - interp_2(sTh[k - 1], sTh[k])) * dzi;
-    }
+    __syncthreads();
   }
 }
 
 template <class M, bool SEED>
 cudaError_t launch_sa(const Geo& geo, const SaArgs& a, cudaStream_t st) {
-  const size_t smem = ((M::exact ? 1 : 4) * geo.n2 * sizeof(double) + 15) / 16 * 16;
+  const size_t smem = (4 * geo.n2 * sizeof(double) + 15) / 16 * 16;
   if (smem > 48 * 1024) {
     const cudaError_t e =
         cudaFuncSetAttribute(thermo_sa_kernel<M, SEED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -308,7 +321,13 @@ cudaError_t launch_dry(const Geo& geo, const DryArgs& a, cudaStream_t st) {
   size_t smem;
   thermo_k::column_launch_shape(geo.n2, 2, &blk, &smem);
   const long long ncols = geo.n0 * geo.n1;
-  thermo_dry_kernel<M><<<ceil_div(ncols, blk.y), blk, smem, st>>>(geo, a, ncols);
+  int dev = 0, sms = 148, per_sm = 1;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, thermo_dry_kernel<M>, (int)(blk.x * blk.y), smem) !=
+          cudaSuccess || per_sm < 1)
+    per_sm = 1;
+  const long long need = ceil_div(ncols, blk.y), most = (long long)sms * per_sm;
+  thermo_dry_kernel<M><<<(unsigned)(need < most ? need : most), blk, smem, st>>>(geo, a, ncols);
   pb_note_launch();
   return cudaGetLastError();
 }
