@@ -15,7 +15,7 @@
 // normalisation.  The loads bound it: 32-level blocks leave few idle lanes
 // on any level count (128 threads along 134 levels left the second block's
 // 122 idle, one load in flight per thread) and 148 chunks give an SM 40 warps
-// at that size.  Measured at 256x256x128 per reduction of one field
+// at that size (296 chunks: 2 us more a reduction).  Measured at 256x256x128 per reduction of one field
 // (81 MB): mean 15.9 us (34.8 with one thread per level and 296
 // chunks), squares 15.2 (39.9), conditional mean (two fields) 28.7 (64.7).
 // Compiled with -fmad=false: the products are rounded before they are added,
@@ -28,6 +28,7 @@ namespace {
 namespace stk {
 
 constexpr int kParts = 148;   // chunks of columns
+constexpr int kSpace = 296;   // partials per level that the workspace holds
 constexpr int kWarps = 8;     // per block
 constexpr int kUnroll = 4;    // columns in flight per warp
 constexpr int kFinal = 256;
@@ -190,7 +191,7 @@ void launch(const A& a, cudaStream_t st) {
 
 extern "C" long long pb_stat_workspace_bytes(const pb_dims* dims) {
   if (pb_check_dims(dims)) return -1;
-  return 2LL * stk::kParts * dims->nlg[2] * (long long)sizeof(double);
+  return 2LL * stk::kSpace * dims->nlg[2] * (long long)sizeof(double);
 }
 
 extern "C" int pb_horizontal_stat(const pb_dims* dims, int kind, const double* v1, const double* v2,
