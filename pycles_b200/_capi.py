@@ -189,9 +189,13 @@ def ptr(t) -> int:
 
 
 def stream_handle(stream=None) -> int:
+    """The CUDA stream of a torch stream, or the current device's current
+    stream (its handle alone: building a torch.cuda.Stream for it took longer
+    than a kernel launch)."""
+    if stream is not None:
+        return stream.cuda_stream
     import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def get_error() -> int:

@@ -47,12 +47,13 @@ class ScalarAdvection:
         if not scal:
             return
         n = len(scal)
-        sp = (ctypes.c_void_p * n)(*[_capi.ptr(PV.field(nm, Gr)) for nm in scal])
-        tp = (ctypes.c_void_p * n)(*[_capi.ptr(PV.tendency(nm, Gr)) for nm in scal])
-        vel = [PV.values[int(PV.velocity_directions[d]) * Gr.dims.npg:] for d in range(3)]
+        va, ta = PV.value_addresses(Gr), PV.tendency_addresses(Gr)
+        sp = (ctypes.c_void_p * n)(*[va[PV.name_index[nm]] for nm in scal])
+        tp = (ctypes.c_void_p * n)(*[ta[PV.name_index[nm]] for nm in scal])
+        vel = [va[int(d)] for d in PV.velocity_directions]
         rc = _capi.load().pb_scalar_advection(
             ctypes.byref(Gr.dims), _capi.ptr(Rs.d_rho0), _capi.ptr(Rs.d_rho0_half), _capi.ptr(Rs.d_alpha0),
-            _capi.ptr(Rs.d_alpha0_half), _capi.ptr(vel[0]), _capi.ptr(vel[1]), _capi.ptr(vel[2]), n, sp, tp,
+            _capi.ptr(Rs.d_alpha0_half), *vel, n, sp, tp,
             _capi.ptr(self.flux) if self.flux is not None else None, self.order, self.precision,
             _capi.stream_handle(stream))
         _capi.check(rc, "pb_scalar_advection")
@@ -81,11 +82,9 @@ class MomentumAdvection:
         self.update_now(Gr, Rs, PV, stream=stream)
 
     def update_now(self, Gr, Rs, PV, DV=None, stream=None):
-        npg = Gr.dims.npg
-        vs = [int(PV.velocity_directions[d]) * npg for d in range(3)]
+        va, ta = PV.value_addresses(Gr), PV.tendency_addresses(Gr)
+        vs = [int(d) for d in PV.velocity_directions]
         rc = _capi.load().pb_momentum_advection(
             ctypes.byref(Gr.dims), _capi.ptr(Rs.d_rho0), _capi.ptr(Rs.d_rho0_half), _capi.ptr(Rs.d_alpha0),
-            _capi.ptr(Rs.d_alpha0_half), _capi.ptr(PV.values[vs[0]:]), _capi.ptr(PV.values[vs[1]:]),
-            _capi.ptr(PV.values[vs[2]:]), _capi.ptr(PV.tendencies[vs[0]:]), _capi.ptr(PV.tendencies[vs[1]:]),
-            _capi.ptr(PV.tendencies[vs[2]:]), self.order, self.precision, _capi.stream_handle(stream))
+            _capi.ptr(Rs.d_alpha0_half), *[va[i] for i in vs], *[ta[i] for i in vs], self.order, self.precision, _capi.stream_handle(stream))
         _capi.check(rc, "pb_momentum_advection")

@@ -763,10 +763,16 @@ inline int march_chunk(long long n_march, long long other_blocks, int per_sm, in
   return best;
 }
 
-template <class K>
-inline int resident_blocks(K kernel, int threads, size_t smem = 0) {
-  int n = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem) != cudaSuccess || n < 1) n = 1;
+// Resident blocks of a kernel per SM: a property of the compiled kernel on
+// this architecture, asked for once (asking took as long as a third of a
+// kernel launch, four times a stage).
+template <auto Kernel>
+inline int resident_blocks(int threads) {
+  static const int n = [threads] {
+    int b = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, Kernel, threads, 0) != cudaSuccess || b < 1) b = 1;
+    return b;
+  }();
   return n;
 }
 
@@ -782,16 +788,16 @@ cudaError_t launch_scalar_group(const Geo& g, ScalarArgs base, double* const* fl
     const long long other = march_blocks(nl1, nl2);
     if constexpr (F32 && NS == 1) {
       if (a.fused) {
-        const int c = march_chunk(nl0, other, resident_blocks(scalar_march_f32<0, ORDER, true>, 128), 2 * R, kChunk, 1, 2);
+        const int c = march_chunk(nl0, other, resident_blocks<scalar_march_f32<0, ORDER, true>>(kMarchThreads), 2 * R, kChunk, 1, 2);
         scalar_march_f32<0, ORDER, true><<<march_grid(nl1, nl2, ceil_div(nl0, c)), kMarchThreads, 0, st>>>(
             g, a, c);
       } else {
-        const int c = march_chunk(nl0, other, resident_blocks(scalar_march_f32<0, ORDER, false>, 128), 2 * R, kChunk, 1, 2);
+        const int c = march_chunk(nl0, other, resident_blocks<scalar_march_f32<0, ORDER, false>>(kMarchThreads), 2 * R, kChunk, 1, 2);
         scalar_march_f32<0, ORDER, false><<<march_grid(nl1, nl2, ceil_div(nl0, c)), kMarchThreads, 0, st>>>(
             g, a, c);
       }
     } else {
-      const int c = march_chunk(nl0, other, resident_blocks(scalar_march<0, ORDER, F32, NS>, 128), 2 * R, kChunk, 1, 2);
+      const int c = march_chunk(nl0, other, resident_blocks<scalar_march<0, ORDER, F32, NS>>(kMarchThreads), 2 * R, kChunk, 1, 2);
       scalar_march<0, ORDER, F32, NS><<<march_grid(nl1, nl2, ceil_div(nl0, c)), kMarchThreads, 0, st>>>(
           g, a, c);
     }
@@ -803,11 +809,11 @@ cudaError_t launch_scalar_group(const Geo& g, ScalarArgs base, double* const* fl
     for (int q = 0; q < NS; ++q) a.flux[q] = flux_dir[1] ? flux_dir[1][q] : nullptr;
     const long long other = march_blocks(nl0, nl2);
     if constexpr (F32 && NS == 1) {
-      const int c = march_chunk(nl1, other, resident_blocks(scalar_march_f32<1, ORDER, false>, 128), 2 * R, kChunk, 1, 2);
+      const int c = march_chunk(nl1, other, resident_blocks<scalar_march_f32<1, ORDER, false>>(kMarchThreads), 2 * R, kChunk, 1, 2);
       scalar_march_f32<1, ORDER, false><<<march_grid(nl0, nl2, ceil_div(nl1, c)), kMarchThreads, 0, st>>>(
           g, a, c);
     } else {
-      const int c = march_chunk(nl1, other, resident_blocks(scalar_march<1, ORDER, F32, NS>, 128), 2 * R, kChunk, 1, 2);
+      const int c = march_chunk(nl1, other, resident_blocks<scalar_march<1, ORDER, F32, NS>>(kMarchThreads), 2 * R, kChunk, 1, 2);
       scalar_march<1, ORDER, F32, NS><<<march_grid(nl0, nl2, ceil_div(nl1, c)), kMarchThreads, 0, st>>>(
           g, a, c);
     }
@@ -878,11 +884,11 @@ cudaError_t launch_momentum(const Geo& g, const MomArgs& a, cudaStream_t st) {
     return cudaGetLastError();
   } else {
   const int c0 = march_chunk(nl0, march_blocks(nl1, nl2),
-                             resident_blocks(momentum_march<0, ORDER, F32>, 128), 2 * R, kChunk, 1, 2);
+                             resident_blocks<momentum_march<0, ORDER, F32>>(kMarchThreads), 2 * R, kChunk, 1, 2);
   momentum_march<0, ORDER, F32><<<march_grid(nl1, nl2, ceil_div(nl0, c0)), kMarchThreads, 0, st>>>(g, a, c0);
   pb_note_launch();
   const int c1 = march_chunk(nl1, march_blocks(nl0, nl2),
-                             resident_blocks(momentum_march<1, ORDER, F32>, 128), 2 * R, kChunk, 1, 2);
+                             resident_blocks<momentum_march<1, ORDER, F32>>(kMarchThreads), 2 * R, kChunk, 1, 2);
   momentum_march<1, ORDER, F32><<<march_grid(nl0, nl2, ceil_div(nl1, c1)), kMarchThreads, 0, st>>>(g, a, c1);
   pb_note_launch();
   momentum_z<ORDER, F32><<<z_grid(nl0, nl1, nl2), kMarchThreads, 0, st>>>(g, a);

@@ -15,9 +15,9 @@
 // normalisation.  The loads bound it: 32-level blocks leave few idle lanes
 // on any level count (128 threads along 134 levels left the second block's
 // 122 idle, one load in flight per thread) and 148 chunks give an SM 40 warps
-// at that size (296 chunks: 2 us more a reduction).  Measured at 256x256x128 per reduction of one field
-// (81 MB): mean 15.9 us (34.8 with one thread per level and 296
-// chunks), squares 15.2 (39.9), conditional mean (two fields) 28.7 (64.7).
+// at that size (296 chunks: 2 us more a reduction).  Measured at 256x256x128
+// per reduction of one field (81 MB): mean 15.9 us (34.8 with one thread per
+// level), squares 15.2 (39.9), conditional mean (two fields) 28.7 (64.7).
 // Compiled with -fmad=false: the products are rounded before they are added,
 // as in the reference's loops.
 #include <string.h>

@@ -54,11 +54,14 @@ class _ForcingBase(ForcingNone):
         f = _capi.PbForcing(self.scheme, self.coriolis_param, float(RS.u0), float(RS.v0),
                             *[_capi.ptr(self.prof[k]) for k in ("ug", "vg", "dtdt", "dqtdt", "subsidence")])
 
+        va, ta = PV.value_addresses(Gr), PV.tendency_addresses(Gr)
+
         def pv(name, arr):
-            return _capi.ptr(arr[PV.get_varshift(Gr, name):]) if name in PV.index_name else None
+            i = PV.name_index.get(name)
+            return None if i is None else arr[i]
 
         def dv(name):
-            return _capi.ptr(DV.values[DV.get_varshift(Gr, name):]) if name in DV.index_name else None
+            return DV.address(name, Gr) if name in DV.name_index else None
 
         umean = vmean = None
         if self.scheme == _capi.PB_FORCING_BOMEX:  # Forcing.pyx:176-177
@@ -69,9 +72,9 @@ class _ForcingBase(ForcingNone):
             vmean = self._stats.HorizontalMean(Gr, PV.field("v", Gr), stream=stream)
         rc = _capi.load().pb_forcing_update(
             ctypes.byref(Gr.dims), ctypes.byref(f), _capi.ptr(RS.d_p0_half), _capi.ptr(umean), _capi.ptr(vmean),
-            pv("u", PV.values), pv("v", PV.values), pv("s", PV.values), pv("qt", PV.values), dv("ql"),
-            dv("temperature"), pv("u", PV.tendencies), pv("v", PV.tendencies), pv("s", PV.tendencies),
-            pv("qt", PV.tendencies), _capi.stream_handle(stream))
+            pv("u", va), pv("v", va), pv("s", va), pv("qt", va), dv("ql"),
+            dv("temperature"), pv("u", ta), pv("v", ta), pv("s", ta),
+            pv("qt", ta), _capi.stream_handle(stream))
         _capi.check(rc, "pb_forcing_update")
 
 

@@ -46,10 +46,11 @@ class PressureSolver:
     def solve(self, Gr, RS, DV, PV, stream=None):
         """PressureSolver.update up to its final ghost fill of PV."""
         nbytes = self._ensure_workspace(Gr, PV.values.device)
-        u, v, w = (PV.field(n, Gr) for n in PV.velocity_names_directional)
+        va = PV.value_addresses(Gr)
+        u, v, w = (va[PV.name_index[n]] for n in PV.velocity_names_directional)
         rc = _capi.load().pb_pressure_solve(
             ctypes.byref(Gr.dims), _capi.ptr(RS.d_rho0), _capi.ptr(RS.d_rho0_half), _capi.ptr(RS.d_alpha0),
-            _capi.ptr(RS.d_alpha0_half), _capi.ptr(u), _capi.ptr(v), _capi.ptr(w),
-            _capi.ptr(DV.field("divergence", Gr)), _capi.ptr(DV.field("dynamic_pressure", Gr)),
+            _capi.ptr(RS.d_alpha0_half), u, v, w,
+            DV.address("divergence", Gr), DV.address("dynamic_pressure", Gr),
             _capi.ptr(self.workspace), nbytes, self.precision, self.refine_sweeps, _capi.stream_handle(stream))
         _capi.check(rc, "pb_pressure_solve")

@@ -43,7 +43,7 @@ class RadiationDyCOMS_RF01(RadiationNone):
         self._z = torch.as_tensor(Gr.z, dtype=torch.float64, device=dev).contiguous()
 
     def update(self, Gr, Ref, PV, DV, Sur=None, TS=None, Pa=None, stream=None):
-        dv = lambda n: _capi.ptr(DV.values[DV.get_varshift(Gr, n):])
+        dv = lambda n: DV.address(n, Gr)  # noqa: E731
         rc = _capi.load().pb_dycoms_radiation(
             ctypes.byref(Gr.dims), ctypes.byref(self.params), _capi.ptr(Ref.d_rho0_half), _capi.ptr(self._z),
             dv("ql"), _capi.ptr(PV.values[PV.get_varshift(Gr, "qt"):]), dv("temperature"),

@@ -72,15 +72,12 @@ class SGS:
     def update(self, Gr, DV, PV, Ke, Sur=None, Pa=None, stream=None):
         """Kinematics' strain-rate magnitude and SGS.update's viscosity and
         diffusivity in one launch."""
-        npg = Gr.dims.npg
-        vel = [PV.values[int(PV.velocity_directions[d]) * npg:] for d in range(3)]
-        bvf = DV.values[DV.get_varshift(Gr, "buoyancy_frequency"):] if "buoyancy_frequency" in DV.index_name \
-            else None
+        va = PV.value_addresses(Gr)
+        bvf = DV.address("buoyancy_frequency", Gr) if "buoyancy_frequency" in DV.name_index else None
         rc = _capi.load().pb_kinematics_sgs(
-            ctypes.byref(Gr.dims), ctypes.byref(self.struct), _capi.ptr(vel[0]), _capi.ptr(vel[1]),
-            _capi.ptr(vel[2]), _capi.ptr(bvf), _capi.ptr(self._zl_half), _capi.ptr(Ke.strain_rate_mag),
-            _capi.ptr(DV.values[DV.get_varshift(Gr, "viscosity"):]),
-            _capi.ptr(DV.values[DV.get_varshift(Gr, "diffusivity"):]), _capi.stream_handle(stream))
+            ctypes.byref(Gr.dims), ctypes.byref(self.struct), *[va[int(d)] for d in PV.velocity_directions], bvf,
+            _capi.ptr(self._zl_half), _capi.ptr(Ke.strain_rate_mag), DV.address("viscosity", Gr),
+            DV.address("diffusivity", Gr), _capi.stream_handle(stream))
         _capi.check(rc, "pb_kinematics_sgs")
 
     def stats_io(self, *args, **kwargs):
@@ -99,13 +96,13 @@ class ScalarDiffusion:
         return
 
     def update(self, Gr, RS, PV, DV, stream=None):
-        npg = Gr.dims.npg
+        va, ta = PV.value_addresses(Gr), PV.tendency_addresses(Gr)
         scal = [i for i in range(PV.nv) if PV.var_type[i] == 1]
         if not scal:
             return
         n = len(scal)
-        vals = (ctypes.c_void_p * n)(*[_capi.ptr(PV.values[i * npg:]) for i in scal])
-        tends = (ctypes.c_void_p * n)(*[_capi.ptr(PV.tendencies[i * npg:]) for i in scal])
+        vals = (ctypes.c_void_p * n)(*[va[i] for i in scal])
+        tends = (ctypes.c_void_p * n)(*[ta[i] for i in scal])
         # flux factor 2 for a TKE variable 'e' (ScalarDiffusion.pyx:122-127)
         factors = (ctypes.c_double * n)(*[2.0 if PV.index_name[i] == "e" else 1.0 for i in scal])
         names = [PV.index_name[i] for i in scal]
@@ -113,7 +110,7 @@ class ScalarDiffusion:
         s_index = names.index("s") if qt_index >= 0 else -1
 
         def dv(name):
-            return _capi.ptr(DV.values[DV.get_varshift(Gr, name):]) if name in DV.index_name else None
+            return DV.address(name, Gr) if name in DV.name_index else None
 
         rc = _capi.load().pb_scalar_diffusion(
             ctypes.byref(Gr.dims), _capi.ptr(RS.d_rho0), _capi.ptr(RS.d_rho0_half), _capi.ptr(RS.d_alpha0_half),
@@ -136,15 +133,13 @@ class MomentumDiffusion:
         return
 
     def update(self, Gr, RS, PV, DV, Ke, stream=None):
-        npg = Gr.dims.npg
-        vel = [int(PV.velocity_directions[d]) * npg for d in range(3)]
-        s = PV.get_varshift(Gr, "s")
+        va, ta = PV.value_addresses(Gr), PV.tendency_addresses(Gr)
+        vel = [int(d) for d in PV.velocity_directions]
         rc = _capi.load().pb_momentum_diffusion(
             ctypes.byref(Gr.dims), _capi.ptr(RS.d_rho0), _capi.ptr(RS.d_rho0_half), _capi.ptr(RS.d_alpha0),
-            _capi.ptr(RS.d_alpha0_half), *[_capi.ptr(PV.values[o:]) for o in vel],
-            _capi.ptr(DV.values[DV.get_varshift(Gr, "viscosity"):]), _capi.ptr(Ke.strain_rate_mag),
-            _capi.ptr(DV.values[DV.get_varshift(Gr, "temperature"):]),
-            *[_capi.ptr(PV.tendencies[o:]) for o in vel], _capi.ptr(PV.tendencies[s:]), _capi.stream_handle(stream))
+            _capi.ptr(RS.d_alpha0_half), *[va[i] for i in vel],
+            DV.address("viscosity", Gr), _capi.ptr(Ke.strain_rate_mag), DV.address("temperature", Gr),
+            *[ta[i] for i in vel], ta[PV.name_index["s"]], _capi.stream_handle(stream))
         _capi.check(rc, "pb_momentum_diffusion")
 
     def stats_io(self, *args, **kwargs):

@@ -53,14 +53,18 @@ class SurfaceBase:
             return
         L = _capi.load()
 
+        va, ta = PV.value_addresses(Gr), PV.tendency_addresses(Gr)
+
         def pv(name):
-            return _capi.ptr(PV.values[PV.get_varshift(Gr, name):]) if name in PV.index_name else None
+            i = PV.name_index.get(name)
+            return None if i is None else va[i]
 
         def pt(name):
-            return _capi.ptr(PV.tendencies[PV.get_varshift(Gr, name):]) if name in PV.index_name else None
+            i = PV.name_index.get(name)
+            return None if i is None else ta[i]
 
         def dv(name):
-            return _capi.ptr(DV.values[DV.get_varshift(Gr, name):]) if name in DV.index_name else None
+            return DV.address(name, Gr) if name in DV.name_index else None
 
         f = _capi.PbSurfaceFields(*[_capi.ptr(self.fields[n]) for n in _capi.SURFACE_FIELDS])
         sc = self._struct(Ref)

@@ -245,7 +245,9 @@ class ThermodynamicsSA:
     def update(self, Gr, RS, PV, DV, stream=None):
         """ThermodynamicsSA.update (ThermodynamicsSA.pyx:176-213) on the GPU."""
         L = _capi.load()
-        f = DV.field
+        npg = int(Gr.dims.npg)
+        f = lambda name: DV.address(name, Gr)  # noqa: E731
+        vals = _capi.ptr(PV.values)
         if self.iter_stats is None or self.iter_stats.device != PV.values.device:
             self.iter_stats = torch.zeros(2, dtype=torch.int64, device=PV.values.device)
         mlp_struct = None
@@ -256,7 +258,6 @@ class ThermodynamicsSA:
             # previous update, then starts their secant from it
             if self.precision != _capi.PB_FP32:
                 raise ValueError("the learned seed belongs to the precision form (gpu.precision = 'fp32')")
-            npg = int(Gr.dims.npg)
             dev = PV.values.device
             if (self._seed_y is None or self._seed_for is not self.mlp or self._seed_y.numel() != npg
                     or self._seed_y.device != dev):
@@ -270,11 +271,10 @@ class ThermodynamicsSA:
             mlp_struct = ctypes.byref(self._mlp_struct)
         table = self.CC.device_table(PV.values.device)
         rc = L.pb_thermo_sa(ctypes.byref(Gr.dims), _capi.ptr(RS.d_p0_half), _capi.ptr(RS.d_alpha0_half),
-                            ctypes.byref(table), _capi.ptr(PV.field("s", Gr)), _capi.ptr(PV.field("qt", Gr)),
-                            _capi.ptr(f("temperature", Gr)), _capi.ptr(f("qv", Gr)), _capi.ptr(f("ql", Gr)),
-                            _capi.ptr(f("qi", Gr)), _capi.ptr(f("alpha", Gr)), _capi.ptr(f("buoyancy", Gr)),
-                            _capi.ptr(f("theta_rho", Gr)), _capi.ptr(f("buoyancy_frequency", Gr)),
-                            _capi.ptr(f("thetali", Gr)), _capi.ptr(PV.tendency("w", Gr)),
+                            ctypes.byref(table), vals + 8 * npg * PV.name_index["s"],
+                            vals + 8 * npg * PV.name_index["qt"], f("temperature"), f("qv"), f("ql"), f("qi"),
+                            f("alpha"), f("buoyancy"), f("theta_rho"), f("buoyancy_frequency"), f("thetali"),
+                            _capi.ptr(PV.tendency("w", Gr)),
                             1 if self.do_qt_clipping else 0, mlp_struct, _capi.ptr(self.iter_stats),
                             self.max_secant_iter, self.precision, _capi.stream_handle(stream))
         _capi.check(rc, "pb_thermo_sa")
@@ -306,10 +306,9 @@ class ThermodynamicsDry:
     def update(self, Gr, RS, PV, DV, stream=None):
         """ThermodynamicsDry.update (ThermodynamicsDry.pyx:105-120) on the GPU."""
         L = _capi.load()
-        f = DV.field
+        f = lambda name: DV.address(name, Gr)  # noqa: E731
         rc = L.pb_thermo_dry(ctypes.byref(Gr.dims), _capi.ptr(RS.d_p0_half), _capi.ptr(RS.d_alpha0_half),
-                             _capi.ptr(PV.field("s", Gr)), _capi.ptr(f("temperature", Gr)),
-                             _capi.ptr(f("alpha", Gr)), _capi.ptr(f("buoyancy", Gr)), _capi.ptr(f("theta", Gr)),
-                             _capi.ptr(f("buoyancy_frequency", Gr)), _capi.ptr(PV.tendency("w", Gr)),
+                             _capi.ptr(PV.field("s", Gr)), f("temperature"), f("alpha"), f("buoyancy"), f("theta"),
+                             f("buoyancy_frequency"), _capi.ptr(PV.tendency("w", Gr)),
                              self.precision, _capi.stream_handle(stream))
         _capi.check(rc, "pb_thermo_dry")

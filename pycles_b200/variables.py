@@ -127,6 +127,17 @@ class PrognosticVariables:
     def get_varshift(self, Gr, name):
         return self.name_index[name] * Gr.dims.npg
 
+    def value_addresses(self, Gr):
+        """Device addresses of the variables' values, in their order (for the
+        call at hand: fused stages swap the buffer, see TimeStepping)."""
+        base, step = _capi.ptr(self.values), 8 * int(Gr.dims.npg)
+        return [base + v * step for v in range(self.nv)]
+
+    def tendency_addresses(self, Gr):
+        """As value_addresses, of `tendencies`, with what reading it does."""
+        base, step = _capi.ptr(self.tendencies), 8 * int(Gr.dims.npg)
+        return [base + v * step for v in range(self.nv)]
+
     def get_variable_array(self, name, Gr):
         i = self.name_index[name]
         npg = Gr.dims.npg
@@ -159,8 +170,8 @@ class PrognosticVariables:
         """Ghost fill of the variables first .. first+count-1 only, of
         PV.values or of another buffer of the same layout."""
         bc = (ctypes.c_double * count)(*[float(b) for b in self.bc_type[first:first + count]])
-        base = (self.values if values is None else values)[first * Gr.dims.npg:]
-        _capi.check(_capi.load().pb_update_all_bcs(ctypes.byref(Gr.dims), _capi.ptr(base), bc, count,
+        base = _capi.ptr(self.values if values is None else values) + 8 * first * int(Gr.dims.npg)
+        _capi.check(_capi.load().pb_update_all_bcs(ctypes.byref(Gr.dims), base, bc, count,
                                                    _capi.stream_handle(stream)), "pb_update_all_bcs")
 
 
@@ -202,6 +213,10 @@ class DiagnosticVariables:
     def field(self, name, Gr):
         i = self.name_index[name]
         return self.values[i * Gr.dims.npg:(i + 1) * Gr.dims.npg]
+
+    def address(self, name, Gr):
+        """Device address of a field (for the call at hand)."""
+        return _capi.ptr(self.values) + 8 * self.name_index[name] * int(Gr.dims.npg)
 
     def get_variable_array(self, name, Gr):
         return self.field(name, Gr).view(*Gr.shape)
