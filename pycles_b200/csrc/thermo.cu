@@ -81,6 +81,7 @@ extern "C" int pb_thermo_sa(const pb_dims* dims, const double* p0_half, const do
   if (!a.err) return PB_ERR_CUDA;
   a.clip = clip_qt;
   a.max_iter = max_iter;
+  a.dzi = 1.0 / geo.dx2;
   const cudaStream_t st = as_stream(stream);
   if (mlp) {
     // the network's output for the cells saturated at the previous call,

@@ -39,6 +39,7 @@ struct SaArgs {
   SeedNet net;
   int clip;
   int max_iter;
+  double dzi;                // 1 / dz
 };
 
 struct DryArgs {
@@ -92,6 +93,13 @@ using thermo_k::SaArgs;
 // (clamped in eos_finish), y refreshed by the network kernel beforehand;
 // a cell whose y is NaN (not saturated at the last refresh) takes the
 // reference's second point.
+//
+// Bound by the latency of the FP64 chains and of the loads at 32 warps per SM
+// (64 registers; 24 warps at 80 without spills and 40 at 48 are both slower).
+// What is live across the secant decides: level values are read where they
+// are used, the w tendency is loaded with the inputs.  Measured: precision
+// form 512x512x256 3.33 ms (3.55 before), seeded 256x256x256 840 us (929),
+// plain form 256x256x128 975 us (998).
 constexpr int kSeg = 30;
 constexpr int kSaThreads = 256;
 
@@ -99,7 +107,7 @@ template <class M, bool SEED>
 __global__ void __launch_bounds__(kSaThreads, 4) thermo_sa_kernel(Geo geo, SaArgs a, long long ncols, int nseg) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int lane = threadIdx.x & 31;
-  const long long n2 = geo.n2;
+  const int n2 = (int)geo.n2;
   // per level: the Exner function and the reciprocals of the Exner function,
   // p0 and alpha0: the divisions by them become multiplications in the
   // precision form and five multiply-adds (div_by, the same quotients) in the
@@ -113,22 +121,29 @@ __global__ void __launch_bounds__(kSaThreads, 4) thermo_sa_kernel(Geo geo, SaArg
     exner_tab[3 * n2 + k] = 1.0 / a.alpha0[k];
   }
   __syncthreads();
-  const long long ntask = ncols * nseg;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-  const double dzi = 1.0 / geo.dx2;
-  unsigned long long my_it = 0, my_sat = 0;
-  for (long long task = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; task < ntask; task += nwarps) {
-    const long long col = task / nseg;
-    const int seg = (int)(task - col * nseg);
-    const long long k = (long long)seg * kSeg - 1 + lane;
+  unsigned int my_it = 0, my_sat = 0;
+  // task = col * nseg + seg, in strides of nwarps (a 64-bit division per task
+  // took 3 to 4 % of the kernel)
+  const long long task0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long dcol = nwarps / nseg;
+  const int dseg = (int)(nwarps - dcol * nseg);
+  long long col = task0 / nseg;
+  int seg = (int)(task0 - col * nseg);
+  for (; col < ncols; col += dcol, seg += dseg) {
+    if (seg >= nseg) {
+      seg -= nseg;
+      if (++col >= ncols) break;
+    }
+    const int k = seg * kSeg - 1 + lane;
     const bool kin = k >= 0 && k < n2;
     const bool own = kin && lane >= 1 && lane <= kSeg;
     const double p0 = kin ? __ldg(a.p0 + k) : 1.0;
-    const double a0 = kin ? __ldg(a.alpha0 + k) : 1.0;
-    const double exner = kin ? exner_tab[k] : 1.0;
     const long long idx = col * n2 + k;  // columns are contiguous: (i*n1 + j)*n2
-    double qt = 0.0, s = 0.0;
+    double qt = 0.0, s = 0.0, wt = 0.0;
     EosStart st{};
+    const bool has_wt = own && k >= 1 && k < n2 - 3;
+    if (has_wt) wt = a.wt[idx];  // here: after the stores below its latency would be exposed
     if (kin) {
       qt = a.qt[idx];
       if (a.clip) {  // clip_qt (Csrc/thermodynamics_sa.h:213-219)
@@ -154,6 +169,9 @@ __global__ void __launch_bounds__(kSaThreads, 4) thermo_sa_kernel(Geo geo, SaArg
       qv = e.qv;
       double al;
       const bool fin = isfinite(T);
+      // (read here: values held across the secant cost spilled registers)
+      const double a0 = __ldg(a.alpha0 + k);
+      const double exner = exner_tab[k];
       if constexpr (M::exact) {
         al = alpha_c(p0, exner_tab[2 * n2 + k], T, qt, qv, fin);
         // bvf_sa first loop (:147-157): theta_rho on k in [1, n2-1)
@@ -170,8 +188,8 @@ __global__ void __launch_bounds__(kSaThreads, 4) thermo_sa_kernel(Geo geo, SaArg
       }
       if (own) {
         if (!fin) pb_flag_at(a.err, PB_ERR_NONFINITE);
-        my_it += (unsigned long long)e.iters;
-        my_sat += e.sat ? 1ull : 0ull;
+        my_it += (unsigned int)e.iters;
+        my_sat += e.sat ? 1u : 0u;
         a.T[idx] = T;
         a.qv[idx] = qv;
         a.ql[idx] = e.ql;
@@ -198,7 +216,7 @@ __global__ void __launch_bounds__(kSaThreads, 4) thermo_sa_kernel(Geo geo, SaArg
     const double b_up = __shfl_down_sync(0xffffffffu, b, 1);
     if (own) {
       // buoyancy_update_sa second loop (:121-130): k in [1, n2-3)
-      if (k >= 1 && k < n2 - 3) a.wt[idx] = a.wt[idx] + interp_2(b, b_up);
+      if (has_wt) a.wt[idx] = wt + interp_2(b, b_up);
       // bvf_sa second loop (:159-180): k in [2, n2-2)
       if (k >= 2 && k < n2 - 2) {
         double bv;
@@ -208,11 +226,11 @@ __global__ void __launch_bounds__(kSaThreads, 4) thermo_sa_kernel(Geo geo, SaArg
           const double rsl = eps_v * pv_star / (p0 - pv_star);
           const double gamma_w = g / cpd * (1.0 / (1.0 - qt)) * (1.0 + Lv * rsl / (Rd * T)) /
                                  (cpm_c(qt) / cpd + Lv * Lv * (eps_v + rsl) * rsl / (cpd * Rd * T * T));
-          const double dTdz = (interp_2(T, T_up) - interp_2(T_dn, T)) * dzi;
-          const double dqtdz = (interp_2(qt, q_up) - interp_2(q_dn, qt)) * dzi;
+          const double dTdz = (interp_2(T, T_up) - interp_2(T_dn, T)) * a.dzi;
+          const double dqtdz = (interp_2(qt, q_up) - interp_2(q_dn, qt)) * a.dzi;
           bv = g / T * (dTdz + gamma_w) * (1.0 + Lv * rsl / (Rd * T)) - dqtdz / (1.0 - qt);
         } else {
-          bv = g / thr * (interp_2(thr, r_up) - interp_2(r_dn, thr)) * dzi;
+          bv = g / thr * (interp_2(thr, r_up) - interp_2(r_dn, thr)) * a.dzi;
         }
         a.bvf[idx] = bv;
       }
@@ -220,13 +238,14 @@ __global__ void __launch_bounds__(kSaThreads, 4) thermo_sa_kernel(Geo geo, SaArg
   }
   if (a.stats) {
     // warp-aggregated secant statistics
+    unsigned long long it = my_it, sat = my_sat;
     for (int off = 16; off > 0; off >>= 1) {
-      my_it += __shfl_down_sync(0xffffffffu, my_it, off);
-      my_sat += __shfl_down_sync(0xffffffffu, my_sat, off);
+      it += __shfl_down_sync(0xffffffffu, it, off);
+      sat += __shfl_down_sync(0xffffffffu, sat, off);
     }
-    if (lane == 0 && (my_it | my_sat)) {
-      atomicAdd(a.stats, my_it);
-      atomicAdd(a.stats + 1, my_sat);
+    if (lane == 0 && (it | sat)) {
+      atomicAdd(a.stats, it);
+      atomicAdd(a.stats + 1, sat);
     }
   }
 }
