@@ -191,6 +191,21 @@ __device__ __forceinline__ double sflux_in(const SArgs& a, const double* phi, do
          a.dxi_div[d];
 }
 
+// Entropy of a cell's vapour less that of its dry air (sw - sd of
+// compute_qt_diffusion_s_source, Csrc/scalar_diffusion.h:70-113).
+__device__ __forceinline__ double source_entropy(const SArgs& a, double qt, long long ijk, int k) {
+  const double qv = a.qv[ijk], T = a.T[ijk], p0 = a.p0_half[k];
+  const double pd = p0 * (1.0 - qt) / (1.0 - qt + eps_vi * qv);
+  const double lT = crm::log(div_by(T, T_tilde, 1.0 / T_tilde));
+  const double sd = sd_tilde + cpd * lT - Rd * crm::log(div_by(pd, p_tilde, 1.0 / p_tilde));
+  const double pv = p0 * eps_vi * qv / (1.0 - qt + eps_vi * qv);
+  const double sv = sv_tilde + cpv * lT - Rv * crm::log(div_by(pv, p_tilde, 1.0 / p_tilde));
+  const double TC = T - 273.15;
+  const double L = (2500.8 - 2.36 * TC + 0.0016 * TC * TC - 0.00006 * TC * TC * TC) * 1000.0;
+  const double sw = sv - (((qt - qv) / qt) * L / T);
+  return sw - sd;
+}
+
 // ScalarDiffusion.update (ScalarDiffusion.pyx:112-150) for one interior
 // cell: per scalar in order, per direction, the flux divergence
 // (scalar_flux_divergence, Csrc/flux_divergence.h:4-32) and, for qt, the
@@ -210,16 +225,7 @@ __global__ void __launch_bounds__(kThreads, 8) scalar_diffusion(SArgs a) {
     const bool src = n == a.qt_index;
     double sw_sd = 0.0;
     if (src) {
-      const double qt = phi[ijk], qv = a.qv[ijk], T = a.T[ijk], p0 = a.p0_half[k];
-      const double pd = p0 * (1.0 - qt) / (1.0 - qt + eps_vi * qv);
-      const double lT = crm::log(div_by(T, T_tilde, 1.0 / T_tilde));
-      const double sd = sd_tilde + cpd * lT - Rd * crm::log(div_by(pd, p_tilde, 1.0 / p_tilde));
-      const double pv = p0 * eps_vi * qv / (1.0 - qt + eps_vi * qv);
-      const double sv = sv_tilde + cpv * lT - Rv * crm::log(div_by(pv, p_tilde, 1.0 / p_tilde));
-      const double TC = T - 273.15;
-      const double L = (2500.8 - 2.36 * TC + 0.0016 * TC * TC - 0.00006 * TC * TC * TC) * 1000.0;
-      const double sw = sv - (((qt - qv) / qt) * L / T);
-      sw_sd = sw - sd;
+      sw_sd = source_entropy(a, phi[ijk], ijk, k);
     }
     for (int d = 0; d < 3; ++d) {
       const long long s = stride_of(g, d);
@@ -237,6 +243,57 @@ __global__ void __launch_bounds__(kThreads, 8) scalar_diffusion(SArgs a) {
     }
     a.tend[n][ijk] = t;
   }
+}
+
+// The same for two scalars (entropy first, then total water with its entropy
+// source if SRC): a face's diffusivity is averaged once for both, and the
+// entropy tendency stays in a register through its source terms instead of
+// three read-modify-writes.  Same operations in the same order per tendency.
+// Measured at 192x192x150 with the source: 207 us against 237.
+template <bool SRC>
+__global__ void __launch_bounds__(kThreads) scalar_diffusion_pair(SArgs a) {
+  const G& g = a.g;
+  int j, k;
+  if (!plane_cell(g.n1 - 2 * g.gw, g.n2 - 2 * g.gw, j, k)) return;
+  j += g.gw;
+  k += g.gw;
+  const int i = g.gw + blockIdx.y;
+  const long long ijk = (long long)i * g.is + (long long)j * g.js + k;
+  const double* p0 = a.phi[0];
+  const double* p1 = a.phi[1];
+  const double f0 = -a.factor[0], f1 = -a.factor[1];
+  const double al = a.alpha0_half[k], rh = a.rho0_half[k];
+  const double Dc = __ldg(a.D + ijk), c0 = __ldg(p0 + ijk), c1 = __ldg(p1 + ijk);
+  double t0 = a.tend[0][ijk], t1 = a.tend[1][ijk];
+  double src[3] = {0.0, 0.0, 0.0};
+  const double ws = SRC ? source_entropy(a, c1, ijk, k) : 0.0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const long long s = stride_of(g, d);
+    const double Dh = 0.5 * (Dc + __ldg(a.D + ijk + s));
+    const double Dl = 0.5 * (__ldg(a.D + ijk - s) + Dc);
+    const double rhoh = d == 2 ? a.rho0[k] : rh, rhol = d == 2 ? a.rho0[k - 1] : rh;
+    const bool floor_face = d == 2 && k == g.gw;  // the face below the first level is 0
+    const double up0 = __ldg(p0 + ijk + s), up1 = __ldg(p1 + ijk + s);
+    const double h0 = f0 * Dh * (up0 - c0) * rhoh * a.dxi_div[d];
+    const double h1 = f1 * Dh * (up1 - c1) * rhoh * a.dxi_div[d];
+    const double l0 = floor_face ? 0.0 : f0 * Dl * (c0 - __ldg(p0 + ijk - s)) * rhol * a.dxi_div[d];
+    const double l1 = floor_face ? 0.0 : f1 * Dl * (c1 - __ldg(p1 + ijk - s)) * rhol * a.dxi_div[d];
+    t0 -= al * (h0 - l0) * g.dxi[d];
+    t1 -= al * (h1 - l1) * g.dxi[d];
+    if constexpr (SRC) {
+      int hi[3] = {i, j, k};
+      hi[d] += 1;
+      const double u1 = sflux(a, p1, a.factor[1], d, ijk + s, hi[0], hi[1], hi[2]);
+      src[d] = ws * al * (u1 - h1) * a.dxi_div[d];
+    }
+  }
+  if constexpr (SRC) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) t0 -= src[d];
+  }
+  a.tend[0][ijk] = t0;
+  a.tend[1][ijk] = t1;
 }
 
 struct MArgs {
@@ -408,7 +465,15 @@ extern "C" int pb_scalar_diffusion(const pb_dims* dims, const double* rho0, cons
   a.qt_index = qt_index;
   a.s_index = qt_index >= 0 ? s_index : -1;
   const dim3 grid = sgsk::plane_grid(dims->n[0], dims->n[1], dims->n[2]);
-  sgsk::scalar_diffusion<<<grid, sgsk::kThreads, 0, as_stream(stream)>>>(a);
+  // the usual pair (s, then qt), on four distinct arrays
+  const bool pair = nscalars == 2 && (qt_index < 0 || qt_index == 1) && a.tend[0] != a.tend[1] &&
+                    a.tend[0] != a.phi[0] && a.tend[0] != a.phi[1] && a.tend[1] != a.phi[0] && a.tend[1] != a.phi[1];
+  if (pair && qt_index == 1)
+    sgsk::scalar_diffusion_pair<true><<<grid, sgsk::kThreads, 0, as_stream(stream)>>>(a);
+  else if (pair)
+    sgsk::scalar_diffusion_pair<false><<<grid, sgsk::kThreads, 0, as_stream(stream)>>>(a);
+  else
+    sgsk::scalar_diffusion<<<grid, sgsk::kThreads, 0, as_stream(stream)>>>(a);
   pb_note_launch();
   PB_LAUNCH_CHECK();
   return PB_OK;
