@@ -126,34 +126,16 @@ struct EosStart {
   bool sat;
 };
 
-// The precision form divides once for the vapour pressure and the exponent
-// (the reciprocal of the product of their denominators) and, where the cell
-// is not saturated, not at all for q_v*: the test qt <= q_v* is made on the
-// products (qv_star_1 is formed for saturated cells only).  The divisions were
-// half of an unsaturated cell's dependent chain, which bounds the kernel.
 template <class M>
 __device__ __forceinline__ EosStart eos_start(const pb_table& LT, double p0, double s, double qt,
                                               unsigned int* err) {
   EosStart e;
-  if constexpr (M::exact) {
-    e.pv_1 = pv_c(p0, qt, qt);
-    e.pd_1 = p0 - e.pv_1;
-    e.T_1 = temperature_no_ql<M>(e.pd_1, e.pv_1, s, qt);
-    const double pv_star_1 = table_lookup(LT, e.T_1, err);
-    e.qv_star_1 = qv_star_c(p0, qt, pv_star_1);
-    e.sat = !(qt <= e.qv_star_1);
-  } else {
-    const double A = 1.0 - qt + eps_vi * qt, B = cpm_c(qt);
-    const double r = 1.0 / (A * B);
-    e.pv_1 = p0 * eps_vi * qt * (r * B);
-    e.pd_1 = p0 - e.pv_1;
-    e.T_1 = T_tilde * M::exp((s - (1.0 - qt) * (sd_tilde - Rd * log_p<M>(e.pd_1)) -
-                              qt * (sv_tilde - Rv * log_p<M>(e.pv_1))) * (r * A));
-    const double pv_star_1 = table_lookup(LT, e.T_1, err);
-    const double num = eps_v * (1.0 - qt) * pv_star_1, den = p0 - pv_star_1;
-    e.sat = den > 0.0 ? !(qt * den <= num) : !(qt <= num / den);
-    e.qv_star_1 = e.sat ? num / den : 0.0;
-  }
+  e.pv_1 = pv_c(p0, qt, qt);
+  e.pd_1 = p0 - e.pv_1;
+  e.T_1 = temperature_no_ql<M>(e.pd_1, e.pv_1, s, qt);
+  const double pv_star_1 = table_lookup(LT, e.T_1, err);
+  e.qv_star_1 = qv_star_c(p0, qt, pv_star_1);
+  e.sat = !(qt <= e.qv_star_1);
   return e;
 }
 
@@ -213,8 +195,7 @@ __device__ __forceinline__ EosOut eos_finish(const pb_table& LT, const EosStart&
   do {
     const double pv_star_2 = table_lookup(LT, T_2, err);
     qv_star_2 = qv_star_c(p0, qt, pv_star_2);
-    // (precision form: the vapour pressure of q_v* is pv* itself, eps_v eps_vi = 1)
-    const double pv_2 = M::exact ? pv_c(p0, qt, qv_star_2) : pv_star_2;
+    const double pv_2 = pv_c(p0, qt, qv_star_2);
     const double pd_2 = p0 - pv_2;
     sigma_2 = qt - qv_star_2;
     const double L_2 = latent_heat(T_2);

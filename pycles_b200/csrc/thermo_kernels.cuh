@@ -98,8 +98,8 @@ using thermo_k::SaArgs;
 // (64 registers; 24 warps at 80 without spills and 40 at 48 are both slower).
 // What is live across the secant decides: level values are read where they
 // are used, the w tendency is loaded with the inputs.  Measured: precision
-// form 512x512x256 3.33 ms (3.55 before), seeded 256x256x256 840 us (929),
-// plain form 256x256x128 975 us (998).
+// form 512x512x256 3.38 ms (3.55 before), seeded 256x256x256 890 us (929),
+// plain form 256x256x128 991 us (998).
 constexpr int kSeg = 30;
 constexpr int kSaThreads = 256;
 
@@ -123,19 +123,12 @@ __global__ void __launch_bounds__(kSaThreads, 4) thermo_sa_kernel(Geo geo, SaArg
   __syncthreads();
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
   unsigned int my_it = 0, my_sat = 0;
-  // task = col * nseg + seg, in strides of nwarps (a 64-bit division per task
-  // took 3 to 4 % of the kernel)
-  const long long task0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long dcol = nwarps / nseg;
-  const int dseg = (int)(nwarps - dcol * nseg);
-  long long col = task0 / nseg;
-  int seg = (int)(task0 - col * nseg);
-  for (; col < ncols; col += dcol, seg += dseg) {
-    if (seg >= nseg) {
-      seg -= nseg;
-      if (++col >= ncols) break;
-    }
-    const int k = seg * kSeg - 1 + lane;
+  const double dzi = a.dzi;
+  const long long ntask = ncols * nseg;
+  for (long long task = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; task < ntask; task += nwarps) {
+    const long long col = task / nseg;
+    const int seg = (int)(task - col * nseg);
+    const long long k = (long long)seg * kSeg - 1 + lane;
     const bool kin = k >= 0 && k < n2;
     const bool own = kin && lane >= 1 && lane <= kSeg;
     const double p0 = kin ? __ldg(a.p0 + k) : 1.0;
@@ -188,7 +181,7 @@ __global__ void __launch_bounds__(kSaThreads, 4) thermo_sa_kernel(Geo geo, SaArg
       }
       if (own) {
         if (!fin) pb_flag_at(a.err, PB_ERR_NONFINITE);
-        my_it += (unsigned int)e.iters;
+        my_it += e.iters;
         my_sat += e.sat ? 1u : 0u;
         a.T[idx] = T;
         a.qv[idx] = qv;
@@ -226,11 +219,11 @@ __global__ void __launch_bounds__(kSaThreads, 4) thermo_sa_kernel(Geo geo, SaArg
           const double rsl = eps_v * pv_star / (p0 - pv_star);
           const double gamma_w = g / cpd * (1.0 / (1.0 - qt)) * (1.0 + Lv * rsl / (Rd * T)) /
                                  (cpm_c(qt) / cpd + Lv * Lv * (eps_v + rsl) * rsl / (cpd * Rd * T * T));
-          const double dTdz = (interp_2(T, T_up) - interp_2(T_dn, T)) * a.dzi;
-          const double dqtdz = (interp_2(qt, q_up) - interp_2(q_dn, qt)) * a.dzi;
+          const double dTdz = (interp_2(T, T_up) - interp_2(T_dn, T)) * dzi;
+          const double dqtdz = (interp_2(qt, q_up) - interp_2(q_dn, qt)) * dzi;
           bv = g / T * (dTdz + gamma_w) * (1.0 + Lv * rsl / (Rd * T)) - dqtdz / (1.0 - qt);
         } else {
-          bv = g / thr * (interp_2(thr, r_up) - interp_2(r_dn, thr)) * a.dzi;
+          bv = g / thr * (interp_2(thr, r_up) - interp_2(r_dn, thr)) * dzi;
         }
         a.bvf[idx] = bv;
       }
