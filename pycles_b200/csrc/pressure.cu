@@ -24,7 +24,8 @@
 //   (remove_mean_u3)           w -= mean[k] on every cell, applied where w is
 //                              read: in the divergence and in the correction
 //   zero_ghosts                divergence ghosts = 0 (the reference zeroes the
-//                              whole array before adding the interior terms)
+//                              whole array before adding the interior terms);
+//                              in the one-GPU solve part of the last ghost_sym
 //   fft_x_fwd                  second_order_divergence (d = 0,1,2 in order)
 //                              + x-FFT of each (j, k) row
 //   fft_y                      y-FFT (forward, or inverse with 1/n1)
@@ -1399,7 +1400,9 @@ __global__ void __launch_bounds__((fft_threads<C, LGN>()), (fft_blocks<C, LGN>()
 }
 
 // ---- pressure ghost fill (sym), communicate_variable on one rank -----------
-__global__ void ghost_sym(Geo g, double* __restrict__ f, long long nghost) {
+// `zero`, if given: a field whose ghosts are set to 0 in the same pass (the
+// divergence, whose ghosts no kernel of the solve reads: one launch less).
+__global__ void ghost_sym(Geo g, double* __restrict__ f, double* __restrict__ zero, long long nghost) {
   const long long gw = g.gw, n0 = g.n0, n1 = g.n1, n2 = g.n2;
   const long long nl0 = n0 - 2 * gw, nl1 = n1 - 2 * gw;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -1412,6 +1415,7 @@ __global__ void ghost_sym(Geo g, double* __restrict__ f, long long nghost) {
     if (k >= n2 - gw) ks = n2 - gw - 1 - (k - (n2 - gw));
     else if (k < gw) ks = gw + (gw - 1 - k);
     f[i * g.is + j * g.js + k] = f[is_ * g.is + js_ * g.js + ks];
+    if (zero != nullptr) zero[i * g.is + j * g.js + k] = 0.0;
   }
 }
 
@@ -1423,10 +1427,18 @@ __global__ void correction(Geo g, const double* __restrict__ p, double* __restri
                            double* __restrict__ w, const double* __restrict__ mean) {
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < g.npg; t += stride) {
-    const long long k = t % g.n2;
-    const long long r = t / g.n2;
-    const long long j = r % g.n1;
-    const long long i = r / g.n1;
+    long long i, j, k;
+    if (g.npg < (1LL << 31)) {  // (two 64-bit divisions per cell were a tenth of the kernel)
+      const unsigned tt = (unsigned)t, r = tt / (unsigned)g.n2, ii = r / (unsigned)g.n1;
+      k = tt - r * (unsigned)g.n2;
+      j = r - ii * (unsigned)g.n1;
+      i = ii;
+    } else {
+      const long long r = t / g.n2;
+      k = t - r * g.n2;
+      i = r / g.n1;
+      j = r - i * g.n1;
+    }
     const double wt = sub_rn(w[t], mean[k]);
     if (i >= g.n0 - 1 || j >= g.n1 - 1 || k >= g.n2 - 1) {
       w[t] = wt;
@@ -1747,10 +1759,6 @@ static int pressure_solve_impl(const pb_dims* dims, const double* rho0, const do
     hmean_final<<<(unsigned)g.n2, 256, 0, st>>>(g, a.partial, a.mean, kPartials, 1.0 / (double)(Ny * Nx));
     pb_note_launch();
   }
-  if (nghost > 0) {
-    zero_ghosts<<<stream_blocks(nghost), 256, 0, st>>>(g, divergence, nghost);
-    pb_note_launch();
-  }
   PB_LAUNCH_CHECK();
 
   int rc;
@@ -1762,14 +1770,14 @@ static int pressure_solve_impl(const pb_dims* dims, const double* rho0, const do
     if ((rc = fft_solve<float2>(g, a, false, false, st))) return rc;
     for (int s = 0; s < refine_sweeps; ++s) {
       if (nghost > 0) {
-        ghost_sym<<<stream_blocks(nghost), 256, 0, st>>>(g, dynamic_pressure, nghost);
+        ghost_sym<<<stream_blocks(nghost), 256, 0, st>>>(g, dynamic_pressure, nullptr, nghost);
         pb_note_launch();
       }
       if ((rc = fft_solve<float2>(g, a, true, true, st))) return rc;
     }
   }
   if (nghost > 0) {
-    ghost_sym<<<stream_blocks(nghost), 256, 0, st>>>(g, dynamic_pressure, nghost);
+    ghost_sym<<<stream_blocks(nghost), 256, 0, st>>>(g, dynamic_pressure, divergence, nghost);
     pb_note_launch();
   }
   correction<<<stream_blocks(g.npg), 256, 0, st>>>(g, dynamic_pressure, u, v, w, a.mean);
