@@ -1428,7 +1428,7 @@ __global__ void correction(Geo g, const double* __restrict__ p, double* __restri
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < g.npg; t += stride) {
     long long i, j, k;
-    if (g.npg < (1LL << 31)) {  // (two 64-bit divisions per cell were a tenth of the kernel)
+    if (g.npg < (1LL << 31)) {
       const unsigned tt = (unsigned)t, r = tt / (unsigned)g.n2, ii = r / (unsigned)g.n1;
       k = tt - r * (unsigned)g.n2;
       j = r - ii * (unsigned)g.n1;
