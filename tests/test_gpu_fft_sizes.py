@@ -1,6 +1,6 @@
-"""The pressure solve on horizontal sizes that are no powers of two (products
-of the factors 2, 3, 5, 7 in every mix of the register radices, larger prime
-factors, primes) and on the short power-of-two lengths, against the FP64
+"""The pressure solve on horizontal sizes that are no powers of two (divisible
+by 4, 5, 6, 8 or 10, by none of them, primes: every number of outputs per
+thread) and on the short power-of-two lengths, against the FP64
 oracle: pressure 1e-11 (the plain form's tolerance) and, in the precision
 form with one refinement sweep, 1e-7 (the level means it cannot correct)."""
 import pytest
