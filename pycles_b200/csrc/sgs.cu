@@ -333,7 +333,11 @@ __device__ __forceinline__ double mflux(const MArgs& a, int i1, int i2, long lon
 // (momentum_flux_divergence, Csrc/flux_divergence.h:34-60), then the
 // entropy source S^2 nu / T (compute_entropy_source,
 // Csrc/momentum_diffusion.h:98-118).
-__global__ void __launch_bounds__(kThreads) momentum_diffusion(MArgs a) {
+// Bound by the latency of its L1 loads: 32 registers, so that 64 warps fill an
+// SM (at 38 it took 2.92 ms at 512x512x256 against 2.64).  256x256x256 678 us
+// (672 with rows of 128 levels, which leave no lane idle there), 192x192x150
+// 242 (252), 300x100x101 140 (155).
+__global__ void __launch_bounds__(kThreads, 16) momentum_diffusion(MArgs a) {
   const G& g = a.g;
   int j, k;
   if (!plane_cell(g.n1 - 2 * g.gw, g.n2 - 2 * g.gw, j, k)) return;
