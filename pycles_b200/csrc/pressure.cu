@@ -1562,10 +1562,25 @@ int ct_lg(long long n) {
   return lg;
 }
 
+// Opt in to more than 48 KiB of shared memory where a launch needs it: the
+// limit holds for the kernel's static part (the forward x-FFT's reciprocals,
+// asked for once: a property of the compiled kernel) and the dynamic part
+// together.  By the dynamic part alone an FP64 solve on 83 or 306 columns
+// along x, of 48,944 and 49,056 bytes, was refused.
+template <auto Kernel>
+static int allow_smem(size_t dynamic) {
+  static const size_t fixed = [] {
+    cudaFuncAttributes at;
+    return cudaFuncGetAttributes(&at, Kernel) == cudaSuccess ? at.sharedSizeBytes : size_t(48 * 1024);
+  }();
+  if (fixed + dynamic > 48 * 1024)
+    PB_CUDA_TRY(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dynamic));
+  return PB_OK;
+}
+
 template <class C, int SRC, int LG>
 static int launch_x_fwd_src(const Geo& g, PArgs& a, dim3 grid, size_t sm, int KC, cudaStream_t st) {
-  if (sm > 48 * 1024)
-    PB_CUDA_TRY(cudaFuncSetAttribute(fft_x_fwd<C, SRC, LG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  if (const int rc = allow_smem<fft_x_fwd<C, SRC, LG>>(sm)) return rc;
   fft_x_fwd<C, SRC, LG><<<grid, fft_threads<C, LG>(), sm, st>>>(g, a, KC);
   return PB_OK;
 }
@@ -1581,8 +1596,7 @@ static int launch_x_fwd(const Geo& g, PArgs& a, int src, dim3 grid, size_t sm, i
 
 template <class C, int DST, int LG>
 static int launch_x_inv_dst(const Geo& g, PArgs& a, dim3 grid, size_t sm, int KC, cudaStream_t st) {
-  if (sm > 48 * 1024)
-    PB_CUDA_TRY(cudaFuncSetAttribute(fft_x_inv<C, DST, LG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  if (const int rc = allow_smem<fft_x_inv<C, DST, LG>>(sm)) return rc;
   fft_x_inv<C, DST, LG><<<grid, fft_threads<C, LG>(), sm, st>>>(g, a, KC);
   return PB_OK;
 }
@@ -1598,14 +1612,13 @@ static int launch_x_inv(const Geo& g, PArgs& a, int dst, dim3 grid, size_t sm, i
 
 template <class C, int LG>
 static int launch_y(const Geo& g, PArgs& a, bool inverse, dim3 grid, size_t sm, int IC, cudaStream_t st) {
-  if (sm > 48 * 1024) {
-    PB_CUDA_TRY(cudaFuncSetAttribute(fft_y<C, false, LG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    PB_CUDA_TRY(cudaFuncSetAttribute(fft_y<C, true, LG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  }
-  if (inverse)
+  if (inverse) {
+    if (const int rc = allow_smem<fft_y<C, true, LG>>(sm)) return rc;
     fft_y<C, true, LG><<<grid, fft_threads<C, LG>(), sm, st>>>(g, a, IC);
-  else
+  } else {
+    if (const int rc = allow_smem<fft_y<C, false, LG>>(sm)) return rc;
     fft_y<C, false, LG><<<grid, fft_threads<C, LG>(), sm, st>>>(g, a, IC);
+  }
   return PB_OK;
 }
 

@@ -3,9 +3,13 @@ by 4, 5, 6, 8 or 10, by none of them, primes: every number of outputs per
 thread) and on the short power-of-two lengths, against the FP64
 oracle: pressure 1e-11 (the plain form's tolerance) and, in the precision
 form with one refinement sweep, 1e-7 (the level means it cannot correct)."""
+import os
+import subprocess
+import sys
+
 import pytest
 
-from helpers import gpu_dv, gpu_sim, host_case, oracle_sim, rel_l2
+from helpers import ROOT, gpu_dv, gpu_sim, host_case, oracle_sim, rel_l2
 from test_gpu_precision import _stir
 
 pytestmark = pytest.mark.gpu
@@ -24,3 +28,27 @@ def test_pressure_on_composite_lengths(nx, ny, precision):
     o.pr_update()
     g.Pr.update(g.Gr, g.RS, g.DV, g.PV)
     assert rel_l2(gpu_dv(g)["dynamic_pressure"], o.dv["dynamic_pressure"]) < (1e-11 if precision == "fp64" else 1e-7)
+
+
+# Widths whose block of lines, twiddles and reciprocals takes just over 48 KiB
+# of shared memory in FP64 (on either side: 71 and 84, 308), each the first
+# solve of its process: a wider solve before it would leave the kernel's limit
+# raised.
+EDGE = """
+import sys
+sys.path.insert(0, {tests!r})
+from test_gpu_fft_sizes import test_pressure_on_composite_lengths as solve
+solve({nx}, 7, "fp64")
+"""
+
+
+@pytest.mark.parametrize("nx", [72, 83, 306])
+def test_first_solve_at_the_shared_memory_limit(nx):
+    code = EDGE.format(tests=os.path.join(ROOT, "tests"), nx=nx)
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("nx", [71, 76, 82, 84, 159, 161, 301, 302, 303, 307, 308])
+def test_widths_around_the_shared_memory_limit(nx):
+    test_pressure_on_composite_lengths(nx, 5, "fp64")
