@@ -58,13 +58,23 @@ __device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(
 // "Computation of elementary functions on the IBM RISC System/6000
 // processor", IBM J. Res. Dev. 34 (1990): with y correctly rounded and q
 // faithful, fma(fma(-b, q, a), y, q) rounds a / b correctly).  Five
-// operations instead of a division sequence with its range tests.  Needs a
-// quotient and residuals in the normal range (|a| above ~1e-290); a zero,
-// an infinite or a NaN gives zero (its sign may be lost) or NaN.
-__device__ __forceinline__ double div_by(double a, double b, double y) {
+// operations instead of a division sequence with its range tests.  For
+// divisors of 2^-60 to 2^1000 in magnitude, where the residuals are exact:
+// quotients of 2^-900 to 2^1022, and 0 (without its sign).  An infinite or
+// NaN dividend or a larger quotient gives NaN, a smaller one may be a unit in
+// the last place off: callers test for these where they can occur.
+__device__ __forceinline__ double div_by_normal(double a, double b, double y) {
   const double q0 = __dmul_rn(a, y);
   const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
   return __fma_rn(__fma_rn(-b, q1, a), y, q1);
+}
+
+// The same for any dividend: the bits of a / b.  (In the thermodynamics and
+// the divergence, with five or six quotients a cell, a test at each cost 8 %
+// of the kernel or more; they test once for all.)
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  const unsigned top = (unsigned)__double2hiint(__dmul_rn(a, y)) & 0x7fffffffu;
+  return top - 0x07b00000u < 0x7fd00000u - 0x07b00000u ? div_by_normal(a, b, y) : a / b;
 }
 
 struct Geo {

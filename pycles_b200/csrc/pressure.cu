@@ -965,9 +965,22 @@ __device__ __forceinline__ double divergence_at(const Geo& g, const PArgs& a, lo
   if constexpr (PLAIN) {
     const double ah = a.alpha0_half[k];
     double d = 0.0;
-    d = add_rn(d, mul_rn(sub_rn(div_by(U[ijk], ah, yh), div_by(U[ijk - g.is], ah, yh)), g.dxi0));
-    d = add_rn(d, mul_rn(sub_rn(div_by(V[ijk], ah, yh), div_by(V[ijk - g.js], ah, yh)), g.dxi1));
-    d = add_rn(d, mul_rn(sub_rn(div_by(wc, a.alpha0[k], yf), div_by(wm, a.alpha0[k - 1], yd)), g.dxi2));
+    d = add_rn(d, mul_rn(sub_rn(div_by_normal(U[ijk], ah, yh), div_by_normal(U[ijk - g.is], ah, yh)), g.dxi0));
+    d = add_rn(d, mul_rn(sub_rn(div_by_normal(V[ijk], ah, yh), div_by_normal(V[ijk - g.js], ah, yh)), g.dxi1));
+    const double dz = mul_rn(sub_rn(div_by_normal(wc, a.alpha0[k], yf), div_by_normal(wm, a.alpha0[k - 1], yd)), g.dxi2);
+    d = add_rn(d, dz);
+    // From 2^-500 up to infinity d is the divisions' d: an infinity or a NaN
+    // among the velocities makes it a NaN here, and quotients too small for
+    // div_by_normal (below 2^-900) are absorbed; so is a smaller d that the
+    // sum before it and a dz of that range cancel to.  Else: the divisions.
+    constexpr unsigned kLow = 0x20b00000u, kInf = 0x7ff00000u;  // high words
+    const unsigned td = (unsigned)__double2hiint(d) & 0x7fffffffu, tz = (unsigned)__double2hiint(dz) & 0x7fffffffu;
+    if (!(td - kLow < kInf - kLow || (td < kLow && tz - kLow < kInf - kLow))) {
+      d = 0.0;
+      d = add_rn(d, mul_rn(sub_rn(U[ijk] / ah, U[ijk - g.is] / ah), g.dxi0));
+      d = add_rn(d, mul_rn(sub_rn(V[ijk] / ah, V[ijk - g.js] / ah), g.dxi1));
+      d = add_rn(d, mul_rn(sub_rn(wc / a.alpha0[k], wm / a.alpha0[k - 1]), g.dxi2));
+    }
     return d;
   } else {
     const double rh = a.rho0_half[k];

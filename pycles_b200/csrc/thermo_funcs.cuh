@@ -34,30 +34,33 @@ __device__ __forceinline__ double qv_star_c(double p0, double qt, double pv) {
 }
 // alpha and buoyancy: buoyancy cancels ~3 digits of alpha, so both keep the
 // reference's separately rounded operations in either form.
-// Their divisors are a level's: ip0 = 1 / p0, ia0 = 1 / alpha0 (div_by).  fin:
-// T is finite; else the results are T's infinity or NaN, as a division's.
+// Their divisors are a level's: ip0 = 1 / p0, ia0 = 1 / alpha0
+// (div_by_normal).  fin: T is finite; else the results are T's infinity or
+// NaN, as a division's.
 __device__ __forceinline__ double alpha_c(double p0, double ip0, double T, double qt, double qv, bool fin) {
-  const double a = div_by(Rd * T, p0, ip0);
+  const double a = div_by_normal(Rd * T, p0, ip0);
   return mul_rn(fin ? a : T, add_rn(sub_rn(1.0, qt), mul_rn(eps_vi, qv)));
 }
 __device__ __forceinline__ double buoyancy_c(double alpha0, double ia0, double alpha, bool fin) {
-  const double b = div_by(mul_rn(g, sub_rn(alpha, alpha0)), alpha0, ia0);
+  const double b = div_by_normal(mul_rn(g, sub_rn(alpha, alpha0)), alpha0, ia0);
   return fin ? b : alpha;
 }
 __device__ __forceinline__ double cpm_c(double qt) { return (1.0 - qt) * cpd + qt * cpv; }
 // log(x / p_tilde) and log(T / T_tilde): the plain form's quotients are the
-// correctly rounded ones, formed with the constants' reciprocals (div_by); the
-// precision form multiplies by them.
+// correctly rounded ones, formed with the constants' reciprocals
+// (div_by_normal: a pressure that is infinite, or a T that is, makes a NaN of
+// the mixture's entropy as with divisions); the precision form multiplies by
+// them.
 template <class M>
 __device__ __forceinline__ double log_p(double p) {
   constexpr double y = 1.0 / p_tilde;
-  if constexpr (M::exact) return M::log(div_by(p, p_tilde, y));
+  if constexpr (M::exact) return M::log(div_by_normal(p, p_tilde, y));
   else return M::log(p * y);
 }
 template <class M>
 __device__ __forceinline__ double log_T(double T) {
   constexpr double y = 1.0 / T_tilde;
-  if constexpr (M::exact) return M::log(div_by(T, T_tilde, y));
+  if constexpr (M::exact) return M::log(div_by_normal(T, T_tilde, y));
   else return M::log(T * y);
 }
 __device__ __forceinline__ double sc_c(double L, double T) { return -L / T; }

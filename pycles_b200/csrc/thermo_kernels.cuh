@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(kSaThreads, 4) thermo_sa_kernel(Geo geo, SaArg
   const int n2 = (int)geo.n2;
   // per level: the Exner function and the reciprocals of the Exner function,
   // p0 and alpha0: the divisions by them become multiplications in the
-  // precision form and five multiply-adds (div_by, the same quotients) in the
+  // precision form and five multiply-adds (div_by_normal, the same quotients) in the
   // plain form
   double* exner_tab = reinterpret_cast<double*>(smraw);  // [4][n2]
   for (int k = threadIdx.x; k < n2; k += blockDim.x) {
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(kSaThreads, 4) thermo_sa_kernel(Geo geo, SaArg
         // bvf_sa first loop (:147-157): theta_rho on k in [1, n2-1)
         if (k >= 1 && k < n2 - 1) {
           const double t = T * (1.0 - qt + eps_vi * qv);
-          thr = fin ? div_by(t, exner, exner_tab[n2 + k]) : t;
+          thr = fin ? div_by_normal(t, exner, exner_tab[n2 + k]) : t;
         }
         // buoyancy_update_sa first loop (:110-119): k in [0, n2-1)
         if (k < n2 - 1) b = buoyancy_c(a0, exner_tab[3 * n2 + k], al, fin);
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(kSaThreads, 4) thermo_sa_kernel(Geo geo, SaArg
         // thetali_update (:185-211) with thetali_c (thermodynamic_functions.h:15-18);
         // without condensate the exponential is exp(-0) = 1 exactly
         const double theta =
-            M::exact ? (fin ? div_by(T, exner, exner_tab[n2 + k]) : T) : T * exner_tab[n2 + k];
+            M::exact ? (fin ? div_by_normal(T, exner, exner_tab[n2 + k]) : T) : T * exner_tab[n2 + k];
         if (e.ql == 0.0 && e.qi == 0.0) {
           a.thetali[idx] = theta * 1.0;
         } else {
@@ -272,10 +272,11 @@ __global__ void __launch_bounds__(1024) thermo_dry_kernel(Geo geo, DryArgs a, lo
     if (active) {
       // eos_c (Csrc/thermodynamics_dry.h:8-10), eos_update (:12-37)
       constexpr double icp = 1.0 / cpd;
-      const double T = T_tilde * (M::exp(div_by(a.s[idx] - sd_tilde + Rd * lp, cpd, icp)));
+      const double x = a.s[idx] - sd_tilde + Rd * lp;
+      const double T = T_tilde * (M::exp(isfinite(x) ? div_by_normal(x, cpd, icp) : x));
       const bool fin = isfinite(T);
       a.T[idx] = T;
-      const double al = mul_rn(fin ? div_by(Rd * T, pd, ipd) : T, 1.0);
+      const double al = mul_rn(fin ? div_by_normal(Rd * T, pd, ipd) : T, 1.0);
       a.alpha[idx] = al;
       // buoyancy_update (:39-73): i < n0-1, j < n1-1, k < n2-1
       double b = 0.0;
@@ -289,7 +290,7 @@ __global__ void __launch_bounds__(1024) thermo_dry_kernel(Geo geo, DryArgs a, lo
       // bvf_dry (:75-110): theta on k in [1, n2)
       double th = 0.0;
       if (k >= 1) {
-        th = fin ? div_by(T, ex, iex) : T;
+        th = fin ? div_by_normal(T, ex, iex) : T;
         a.theta[idx] = th;
       }
       sTh[k] = th;
