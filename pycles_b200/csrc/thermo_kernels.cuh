@@ -246,41 +246,50 @@ __global__ void __launch_bounds__(kSaThreads, 4) thermo_sa_kernel(Geo geo, SaArg
 // ThermodynamicsDry.update (ThermodynamicsDry.pyx:105-120).  A thread keeps
 // one level: what depends on the level alone (log(p0 / p_tilde), the Exner
 // function, the divisors' reciprocals) is formed once and the block walks over
-// columns, resident blocks only.  One column per block evaluated the level's
-// log and pow for every cell: 266 us at 256x256x128 (FP64), 223 now.
+// columns, resident blocks only.  The vertical neighbours' theta and buoyancy
+// come through shared memory, in two buffers taken in turn, so that one
+// barrier a column set is enough, and the w tendency is loaded before it.
+// Measured at 160x160 columns, one column per block with the level's log and
+// pow for every cell / walking with one buffer and two barriers / now: 96
+// levels FP64 90 / 93 / 78 us, precision form 82 / 87 / 68; 300 levels 220 /
+// 199 / 159 and 201 / 185 / 132.
 template <class M>
 __global__ void __launch_bounds__(1024) thermo_dry_kernel(Geo geo, DryArgs a, long long ncols) {
   extern __shared__ __align__(16) unsigned char smraw[];
   double* sm = reinterpret_cast<double*>(smraw);
   const int kpad = blockDim.x;
   const int k = threadIdx.x;
-  const long long n2 = geo.n2;
-  double* sTh = sm + (size_t)threadIdx.y * 2 * kpad;
-  double* sB = sTh + kpad;
+  const int n2 = (int)geo.n2;
+  double* sTh = sm + (size_t)threadIdx.y * 4 * kpad;  // this buffer's theta, then its buoyancy
+  double* other = sTh + 2 * kpad;
   const bool kin = k < n2;
   const double pd = kin ? a.pd[k] : 1.0, a0 = kin ? a.alpha0[k] : 1.0;
   const double lp = M::log(pd / p_tilde), ex = pow(pd / p_tilde, kappa);
   const double ipd = 1.0 / pd, ia0 = 1.0 / a0, iex = 1.0 / ex;
   const double dzi = 1.0 / geo.dx2;
-  for (long long c0 = (long long)blockIdx.x * blockDim.y; c0 < ncols; c0 += (long long)gridDim.x * blockDim.y) {
-    const long long col = c0 + threadIdx.y;
-    const bool active = col < ncols && kin;
-    const long long i = col / geo.n1;
-    const long long j = col - i * geo.n1;
-    const long long idx = col * n2 + k;
-    const bool bij = (i < geo.n0 - 1) && (j < geo.n1 - 1);
+  // (fields of 2^32 columns do not fit the device)
+  const unsigned n1 = (unsigned)geo.n1, nc = (unsigned)ncols, step = gridDim.x * blockDim.y;
+  for (unsigned c0 = blockIdx.x * blockDim.y; c0 < nc; c0 += step) {
+    const unsigned col = c0 + threadIdx.y;
+    const bool active = col < nc && kin;
+    const unsigned i = col / n1, j = col - i * n1;
+    const long long idx = (long long)col * n2 + k;
+    const bool bij = (i + 1 < (unsigned)geo.n0) && (j + 1 < n1);
+    double* sB = sTh + kpad;
+    const bool has_wt = active && bij && k < n2 - 1;
+    double wt = 0.0, b = 0.0, th = 0.0;
     if (active) {
       // eos_c (Csrc/thermodynamics_dry.h:8-10), eos_update (:12-37)
       constexpr double icp = 1.0 / cpd;
       const double x = a.s[idx] - sd_tilde + Rd * lp;
+      if (has_wt) wt = a.wt[idx];
       const double T = T_tilde * (M::exp(isfinite(x) ? div_by_normal(x, cpd, icp) : x));
       const bool fin = isfinite(T);
       a.T[idx] = T;
       const double al = mul_rn(fin ? div_by_normal(Rd * T, pd, ipd) : T, 1.0);
       a.alpha[idx] = al;
       // buoyancy_update (:39-73): i < n0-1, j < n1-1, k < n2-1
-      double b = 0.0;
-      if (bij && k < n2 - 1) {
+      if (has_wt) {
         b = buoyancy_c(a0, ia0, al, fin);
         a.buoy[idx] = b;
       } else if (bij) {
@@ -288,7 +297,6 @@ __global__ void __launch_bounds__(1024) thermo_dry_kernel(Geo geo, DryArgs a, lo
       }
       sB[k] = b;
       // bvf_dry (:75-110): theta on k in [1, n2)
-      double th = 0.0;
       if (k >= 1) {
         th = fin ? div_by_normal(T, ex, iex) : T;
         a.theta[idx] = th;
@@ -296,12 +304,12 @@ __global__ void __launch_bounds__(1024) thermo_dry_kernel(Geo geo, DryArgs a, lo
       sTh[k] = th;
     }
     __syncthreads();
-    if (active) {
-      if (bij && k < n2 - 1) a.wt[idx] += interp_2(sB[k], sB[k + 1]);
-      if (k >= 2 && k < n2 - 1)
-        a.bvf[idx] = g / sTh[k] * (interp_2(sTh[k], sTh[k + 1]) - interp_2(sTh[k - 1], sTh[k])) * dzi;
-    }
-    __syncthreads();
+    if (has_wt) a.wt[idx] = wt + interp_2(b, sB[k + 1]);
+    if (active && k >= 2 && k < n2 - 1)
+      a.bvf[idx] = g / th * (interp_2(th, sTh[k + 1]) - interp_2(sTh[k - 1], th)) * dzi;
+    double* t = sTh;
+    sTh = other;
+    other = t;
   }
 }
 
@@ -328,18 +336,31 @@ cudaError_t launch_sa(const Geo& geo, const SaArgs& a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+// Resident blocks of the dry kernel per SM, by the block's warps (its shared
+// memory is 32 bytes a thread): a property of the compiled kernel on this
+// architecture, asked for once for each.
+template <class M>
+int dry_blocks_per_sm(int threads, size_t smem) {
+  static std::atomic<int> known[33];
+  std::atomic<int>& slot = known[threads / 32];
+  int n = slot.load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, thermo_dry_kernel<M>, threads, smem) != cudaSuccess || n < 1)
+      return 1;
+    slot.store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
 template <class M>
 cudaError_t launch_dry(const Geo& geo, const DryArgs& a, cudaStream_t st) {
   dim3 blk;
   size_t smem;
-  thermo_k::column_launch_shape(geo.n2, 2, &blk, &smem);
+  thermo_k::column_launch_shape(geo.n2, 4, &blk, &smem);
   const long long ncols = geo.n0 * geo.n1;
-  int dev = 0, sms = 148, per_sm = 1;
+  int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, thermo_dry_kernel<M>, (int)(blk.x * blk.y), smem) !=
-          cudaSuccess || per_sm < 1)
-    per_sm = 1;
-  const long long need = ceil_div(ncols, blk.y), most = (long long)sms * per_sm;
+  const long long need = ceil_div(ncols, blk.y), most = (long long)sms * dry_blocks_per_sm<M>((int)(blk.x * blk.y), smem);
   thermo_dry_kernel<M><<<(unsigned)(need < most ? need : most), blk, smem, st>>>(geo, a, ncols);
   pb_note_launch();
   return cudaGetLastError();
