@@ -256,7 +256,9 @@ __device__ __forceinline__ void split_idx(int e, int d, int& q, int& r) {
 // memory, conjugated for the inverse.  One output per thread, with its own
 // input and global twiddle loads and index, ran at a tenth of the FP64 pipe.
 // Measured, one y-FFT: 36 us at 96x96x150 (FP64; 113 before), 37 at
-// 150x120x90 (FP32; 105 before).
+// 150x120x90 (FP32; 105 before); lengths without such a divisor (dft_any), one
+// solve: 127x127x40 275 us (FP64; 608), FP32 form 410 (506), 997x48x30 1348
+// (3167) and 2068 (3883).
 __device__ __forceinline__ double mul_add(double a, double b, double c, double d, double acc) {  // acc + (a b + c d)
   return __dadd_rn(acc, __fma_rn(a, b, __dmul_rn(c, d)));
 }
@@ -311,10 +313,10 @@ __device__ __forceinline__ void dft_rows(const C* in, C* out, C* table, int nlin
   __syncthreads();
 }
 
-// Any N: G = N / TM rounded up, an index per output.
-template <class C, bool INV>
+// Any N: G = N / TM rounded up, an index per output.  An output past the last
+// (m = m0 + q G >= N) computes number m - N and is not stored.
+template <class C, int TM, bool INV>
 __device__ __forceinline__ void dft_any(const C* in, C* out, C* stw, int nlines, int N, const C* __restrict__ tw) {
-  constexpr int TM = 6;
   const int ld = line_ld(N), G = (N + TM - 1) / TM;
   for (int m = threadIdx.x; m < N; m += kFftThreads) {
     C w = tw[m];
@@ -325,11 +327,13 @@ __device__ __forceinline__ void dft_any(const C* in, C* out, C* stw, int nlines,
   for (int e = threadIdx.x; e < nlines * G; e += kFftThreads) {
     const int m0 = e / nlines, l = e - m0 * nlines;
     C acc[TM];
-    int idx[TM];
+    int idx[TM], step[TM];
 #pragma unroll
     for (int q = 0; q < TM; ++q) {
+      const int m = m0 + q * G;
       acc[q] = czero<C>();
       idx[q] = 0;
+      step[q] = m < N ? m : m - N;
     }
     const C* line = in + l * ld;
 #pragma unroll 4
@@ -338,10 +342,7 @@ __device__ __forceinline__ void dft_any(const C* in, C* out, C* stw, int nlines,
 #pragma unroll
       for (int q = 0; q < TM; ++q) {
         dft_term<C, INV>(acc[q], stw[idx[q]], x);
-        // an output past the last, m = m0 + q G >= N, only keeps its index
-        // in range: m < N + TM, so two steps back always do
-        idx[q] += m0 + q * G;
-        if (idx[q] >= N) idx[q] -= N;
+        idx[q] += step[q];
         if (idx[q] >= N) idx[q] -= N;
       }
     }
@@ -363,7 +364,8 @@ __device__ __forceinline__ void dft_lines(const C* in, C* out, C* table, int nli
     case 6: dft_rows<C, 6, INV>(in, out, table, nlines, N, tw); break;
     case 8: dft_rows<C, 8, INV>(in, out, table, nlines, N, tw); break;
     case 10: dft_rows<C, 10, INV>(in, out, table, nlines, N, tw); break;
-    default: dft_any<C, INV>(in, out, table, nlines, N, tw); break;
+    case 2: dft_any<C, 2, INV>(in, out, table, nlines, N, tw); break;
+    default: dft_any<C, 6, INV>(in, out, table, nlines, N, tw); break;
   }
 }
 
@@ -1489,10 +1491,13 @@ bool fft_sizes_ok(const pb_dims* d) {
 // of N among the built ones that gives all outputs of a block's lines a
 // thread in one round, else the largest; the twiddle table (TM N values) has
 // to leave room for two blocks of 80 KiB of lines per SM (FP64) or three of
-// 48 KiB (FP32).  0: none divides N (or N is a power of two), dft_any.
+// 48 KiB (FP32).  Where none divides N, dft_any: with 2 outputs per thread if
+// that is one round (on few points the length of a thread's chain counts: a
+// solve of 27x27x40 68 us, 76 with 6 outputs; FP32 form 113, 133), else with
+// 6 (returned as 0, as for powers of two).
 int direct_outputs(long long N, int lines, size_t elem) {
   if (pow2(N)) return 0;
-  int best = 0;
+  int best = lines * ((N + 1) / 2) <= kFftThreads ? 2 : 0;
   const int built[] = {4, 5, 6, 8, 10};
   for (int tm : built) {
     if (N % tm != 0 || tm * N * (long long)elem > 24 * 1024) continue;
@@ -1505,7 +1510,7 @@ int direct_outputs(long long N, int lines, size_t elem) {
 size_t fft_smem(long long N, int lines, size_t elem) {
   if (pow2(N)) return (size_t)line_ld((int)N) * lines * elem;
   const int tm = direct_outputs(N, lines, elem);  // a second set of lines and the twiddles
-  return (2 * (size_t)line_ld((int)N) * lines + (size_t)N * (tm > 0 ? tm : 1)) * elem;
+  return (2 * (size_t)line_ld((int)N) * lines + (size_t)N * (tm > 2 ? tm : 1)) * elem;
 }
 
 // Lines per FFT block: a power of two, up to 16, with nlines * N <=

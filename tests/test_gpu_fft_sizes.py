@@ -1,8 +1,11 @@
 """The pressure solve on horizontal sizes that are no powers of two (divisible
 by 4, 5, 6, 8 or 10, by none of them, primes: every number of outputs per
-thread) and on the short power-of-two lengths, against the FP64
-oracle: pressure 1e-11 (the plain form's tolerance) and, in the precision
-form with one refinement sweep, 1e-7 (the level means it cannot correct)."""
+thread; up to 1000 points: blocks of 16, 8, 4 and 2 lines, divisors whose
+twiddle table would be too large) and on the short power-of-two lengths,
+against the FP64 oracle: pressure 1e-11 (the plain form's tolerance) and, in
+the precision form with one refinement sweep, 1e-7 (the level means it cannot
+correct; beyond 150 points in proportion to the points, the bound on the
+rounding of an FP32 sum)."""
 import os
 import subprocess
 import sys
@@ -20,6 +23,10 @@ SIZES = [(96, 90), (150, 12), (100, 21), (49, 35), (22, 26), (97, 6), (18, 54), 
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 @pytest.mark.parametrize("nx,ny", SIZES)
 def test_pressure_on_composite_lengths(nx, ny, precision):
+    _solve_and_compare(nx, ny, 1e-11 if precision == "fp64" else 1e-7, precision)
+
+
+def _solve_and_compare(nx, ny, tol, precision):
     nl, rs, f = host_case(case="bomex", nx=nx, ny=ny, nz=7, dx=100.0, dy=100.0, dz=40.0)
     f = _stir(f)
     o, g = oracle_sim(nl, rs, f), gpu_sim(nl, rs, f, precision=precision)
@@ -27,7 +34,16 @@ def test_pressure_on_composite_lengths(nx, ny, precision):
     g.PV.Update_all_bcs(g.Gr)
     o.pr_update()
     g.Pr.update(g.Gr, g.RS, g.DV, g.PV)
-    assert rel_l2(gpu_dv(g)["dynamic_pressure"], o.dv["dynamic_pressure"]) < (1e-11 if precision == "fp64" else 1e-7)
+    assert rel_l2(gpu_dv(g)["dynamic_pressure"], o.dv["dynamic_pressure"]) < tol
+
+
+LONG = [(31, 33), (7, 29), (11, 304), (389, 4), (5, 511), (720, 5), (997, 6), (6, 1000)]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("nx,ny", LONG)
+def test_pressure_on_long_and_short_lengths(nx, ny, precision):
+    _solve_and_compare(nx, ny, 1e-11 if precision == "fp64" else 1e-7 * max(1.0, max(nx, ny) / 150.0), precision)
 
 
 # Widths whose block of lines, twiddles and reciprocals takes just over 48 KiB
