@@ -111,13 +111,25 @@ inline long long march_blocks(long long n_other, long long nz) {
 // warp takes 32 consecutive faces, the first only for the face below the
 // second's cell; every later lane owns the cell below its face.  By rows: 31
 // cells of a row to a warp; where that leaves more than 1/16 of the lanes
-// idle, 32 consecutive ones of the (nz + 1) faces of the rows of an x plane
-// (a row's lowest face owns no cell).  Measured, scalars, FP64: 128 levels
-// (17% idle) 220 us by rows, 187 flat, at 256x256; 150 levels (3%) 42 and 45
-// at 96x96; FP32, 256 levels (8%) 667 and 638 at 512x512.
+// idle (z_flat), 32 consecutive ones of the (nz + 1) faces of the rows of an
+// x plane (a row's lowest face owns no cell).  Measured, scalars, FP64: 128
+// levels (17% idle) 220 us by rows, 187 flat, at 256x256; 150 levels (3%) 42
+// and 45 at 96x96; FP32, 256 levels (8%) 667 and 638 at 512x512.  ROWS: the
+// map by rows, known at compile time: with both maps in the kernel a thread of
+// two faces took 3.7% longer (FP64 WENO7, 160x160x300: 235 us, 226).  The
+// other instance, launched for the flat map, keeps the choice at run time:
+// with the flat map alone the compiler's allocation made it 0.7% slower.
+inline bool z_flat(long long nz) { return rows_waste((unsigned)nz, 31, 16); }
+template <bool ROWS>
 __device__ __forceinline__ bool z_face(const Geo& g, int lane, long long& j, long long& f, bool& cell) {
-  const unsigned nz = (unsigned)(g.n2 - 2 * g.gw), nj = (unsigned)(g.n1 - 2 * g.gw);
   const unsigned w = threadIdx.x >> 5;
+  if constexpr (ROWS) {
+    j = g.gw + (long long)blockIdx.y * (kMarchThreads / 32) + w;
+    f = g.gw + (long long)blockIdx.x * 31 - 1 + lane;
+    cell = f <= g.n2 - g.gw - 1 && lane > 0;
+    return f <= g.n2 - g.gw - 1;
+  }
+  const unsigned nz = (unsigned)(g.n2 - 2 * g.gw), nj = (unsigned)(g.n1 - 2 * g.gw);
   unsigned q, r;
   if (rows_waste(nz, 31, 16)) {
     const unsigned t = (blockIdx.x * (kMarchThreads / 32) + w) * 31 + lane;
@@ -135,8 +147,8 @@ __device__ __forceinline__ bool z_face(const Geo& g, int lane, long long& j, lon
 }
 inline dim3 z_grid(long long nl0, long long nl1, long long nl2) {
   constexpr int W = kMarchThreads / 32;
-  return rows_waste((unsigned)nl2, 31, 16) ? dim3(ceil_div(nl1 * (nl2 + 1), 31 * W), 1, (unsigned)nl0)
-                                           : dim3(ceil_div(nl2, 31), ceil_div(nl1, W), (unsigned)nl0);
+  return z_flat(nl2) ? dim3(ceil_div(nl1 * (nl2 + 1), 31 * W), 1, (unsigned)nl0)
+                     : dim3(ceil_div(nl2, 31), ceil_div(nl1, W), (unsigned)nl0);
 }
 
 // ---------------------------------------------------------------------------
@@ -194,13 +206,14 @@ __global__ void __launch_bounds__(kMarchThreads) scalar_march(Geo g, ScalarArgs 
 // ---------------------------------------------------------------------------
 // scalars, z direction
 // ---------------------------------------------------------------------------
-template <int ORDER, bool F32, int NS>
+template <int ORDER, bool F32, int NS, bool ROWS>
 __global__ void __launch_bounds__(kMarchThreads) scalar_z(Geo g, ScalarArgs a) {
   constexpr int R = St<ORDER>::R;
   const int lane = threadIdx.x & 31;
   long long j, f;
   bool cell;
-  const bool valid = z_face(g, lane, j, f, cell);
+  const bool valid = z_face<ROWS>(g, lane, j, f, cell);
+  if (ROWS && j >= g.n1 - g.gw) return;  // whole warps
   const long long i = g.gw + (long long)blockIdx.z;
   const long long col = i * g.is + j * g.js;
   const double dzi = g.dxi2;
@@ -301,14 +314,15 @@ __global__ void __launch_bounds__(kMarchThreads) scalar_march_f32(Geo g, ScalarA
 // applied here, the new value written to a.vnew (the stencils of other
 // warps still read the current values) and, at stage 0, the copy; the
 // tendency is not stored.
-template <int ORDER, bool RK>
+template <int ORDER, bool RK, bool ROWS>
 __global__ void __launch_bounds__(kMarchThreads) scalar_z_f32(Geo g, ScalarArgs a) {
   constexpr int R = St<ORDER>::R;
   constexpr int ND = 2 * R - 1;
   const int lane = threadIdx.x & 31;
   long long j, f;
   bool cell;
-  const bool valid = z_face(g, lane, j, f, cell);
+  const bool valid = z_face<ROWS>(g, lane, j, f, cell);
+  if (ROWS && j >= g.n1 - g.gw) return;  // whole warps
   const long long i = g.gw + (long long)blockIdx.z;
   const long long col = i * g.is + j * g.js;
   double F = 0.0, val = 0.0;
@@ -426,12 +440,13 @@ __global__ void __launch_bounds__(kMarchThreads) momentum_march(Geo g, MomArgs a
 // ---------------------------------------------------------------------------
 // momentum, z direction (advecting velocity = w)
 // ---------------------------------------------------------------------------
-template <int ORDER, bool F32>
+template <int ORDER, bool F32, bool ROWS>
 __global__ void __launch_bounds__(kMarchThreads) momentum_z(Geo g, MomArgs a) {
   const int lane = threadIdx.x & 31;
   long long j, f;
   bool cell;
-  const bool valid = z_face(g, lane, j, f, cell);
+  const bool valid = z_face<ROWS>(g, lane, j, f, cell);
+  if (ROWS && j >= g.n1 - g.gw) return;  // whole warps
   const long long i = g.gw + (long long)blockIdx.z;
   const long long idx = i * g.is + j * g.js + f;
   const double dzi = g.dxi2;
@@ -824,13 +839,20 @@ cudaError_t launch_scalar_group(const Geo& g, ScalarArgs base, double* const* fl
     a.vel = vel[2];
     for (int q = 0; q < NS; ++q) a.flux[q] = flux_dir[2] ? flux_dir[2][q] : nullptr;
     const dim3 grd = z_grid(nl0, nl1, nl2);
+    const bool rows = !z_flat(nl2);
     if constexpr (F32 && NS == 1) {
-      if (a.fused)
-        scalar_z_f32<ORDER, true><<<grd, kMarchThreads, 0, st>>>(g, a);
+      if (a.fused && rows)
+        scalar_z_f32<ORDER, true, true><<<grd, kMarchThreads, 0, st>>>(g, a);
+      else if (a.fused)
+        scalar_z_f32<ORDER, true, false><<<grd, kMarchThreads, 0, st>>>(g, a);
+      else if (rows)
+        scalar_z_f32<ORDER, false, true><<<grd, kMarchThreads, 0, st>>>(g, a);
       else
-        scalar_z_f32<ORDER, false><<<grd, kMarchThreads, 0, st>>>(g, a);
+        scalar_z_f32<ORDER, false, false><<<grd, kMarchThreads, 0, st>>>(g, a);
+    } else if (rows) {
+      scalar_z<ORDER, F32, NS, true><<<grd, kMarchThreads, 0, st>>>(g, a);
     } else {
-      scalar_z<ORDER, F32, NS><<<grd, kMarchThreads, 0, st>>>(g, a);
+      scalar_z<ORDER, F32, NS, false><<<grd, kMarchThreads, 0, st>>>(g, a);
     }
     pb_note_launch();
   }
@@ -891,7 +913,11 @@ cudaError_t launch_momentum(const Geo& g, const MomArgs& a, cudaStream_t st) {
                              resident_blocks<momentum_march<1, ORDER, F32>>(kMarchThreads), 2 * R, kChunk, 1, 2);
   momentum_march<1, ORDER, F32><<<march_grid(nl0, nl2, ceil_div(nl1, c1)), kMarchThreads, 0, st>>>(g, a, c1);
   pb_note_launch();
-  momentum_z<ORDER, F32><<<z_grid(nl0, nl1, nl2), kMarchThreads, 0, st>>>(g, a);
+  const dim3 gz = z_grid(nl0, nl1, nl2);
+  if (!z_flat(nl2))
+    momentum_z<ORDER, F32, true><<<gz, kMarchThreads, 0, st>>>(g, a);
+  else
+    momentum_z<ORDER, F32, false><<<gz, kMarchThreads, 0, st>>>(g, a);
   pb_note_launch();
   return cudaGetLastError();
   }
