@@ -69,12 +69,12 @@ __device__ __forceinline__ double div_by_normal(double a, double b, double y) {
   return __fma_rn(__fma_rn(-b, q1, a), y, q1);
 }
 
-// The same for any dividend: the bits of a / b.  (In the thermodynamics and
-// the divergence, with five or six quotients a cell, a test at each cost 8 %
-// of the kernel or more; they test once for all.)
-__device__ __forceinline__ double div_by(double a, double b, double y) {
-  const unsigned top = (unsigned)__double2hiint(__dmul_rn(a, y)) & 0x7fffffffu;
-  return top - 0x07b00000u < 0x7fd00000u - 0x07b00000u ? div_by_normal(a, b, y) : a / b;
+// Whether a result of div_by_normal is the quotient: it lies within that range
+// (no quotient outside comes out within it).  Else the caller divides.  With
+// three to six quotients a cell (thermodynamics, divergence, entropy source) a
+// test at each cost 2 to 20 % of the kernel: they test once for all.
+__device__ __forceinline__ bool quotient_normal(double q) {
+  return ((unsigned)__double2hiint(q) & 0x7fffffffu) - 0x07b00000u < 0x7fd00000u - 0x07b00000u;
 }
 
 struct Geo {

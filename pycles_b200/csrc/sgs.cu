@@ -196,10 +196,19 @@ __device__ __forceinline__ double sflux_in(const SArgs& a, const double* phi, do
 __device__ __forceinline__ double source_entropy(const SArgs& a, double qt, long long ijk, int k) {
   const double qv = a.qv[ijk], T = a.T[ijk], p0 = a.p0_half[k];
   const double pd = p0 * (1.0 - qt) / (1.0 - qt + eps_vi * qv);
-  const double lT = crm::log(div_by(T, T_tilde, 1.0 / T_tilde));
-  const double sd = sd_tilde + cpd * lT - Rd * crm::log(div_by(pd, p_tilde, 1.0 / p_tilde));
   const double pv = p0 * eps_vi * qv / (1.0 - qt + eps_vi * qv);
-  const double sv = sv_tilde + cpv * lT - Rv * crm::log(div_by(pv, p_tilde, 1.0 / p_tilde));
+  double rT = div_by_normal(T, T_tilde, 1.0 / T_tilde);
+  double rd = div_by_normal(pd, p_tilde, 1.0 / p_tilde);
+  double rv = div_by_normal(pv, p_tilde, 1.0 / p_tilde);
+  // one test for the three: a zero (no vapour), an infinity, a NaN
+  if (!(quotient_normal(rT) && quotient_normal(rd) && quotient_normal(rv))) {
+    rT = T / T_tilde;
+    rd = pd / p_tilde;
+    rv = pv / p_tilde;
+  }
+  const double lT = crm::log(rT);
+  const double sd = sd_tilde + cpd * lT - Rd * crm::log(rd);
+  const double sv = sv_tilde + cpv * lT - Rv * crm::log(rv);
   const double TC = T - 273.15;
   const double L = (2500.8 - 2.36 * TC + 0.0016 * TC * TC - 0.00006 * TC * TC * TC) * 1000.0;
   const double sw = sv - (((qt - qv) / qt) * L / T);

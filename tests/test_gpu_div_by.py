@@ -1,9 +1,10 @@
 """Division by a divisor whose reciprocal is kept (csrc/pb_common.cuh), over the
 divisors that the kernels use and around powers of two, for quotients of every
-magnitude, near half-way cases, zeros, infinities and NaNs: div_by has the
-bits of `/` on all, div_by_normal on the range that it states; and the callers
-of the latter on unusual inputs: the pressure solve's divergence and the dry
-thermodynamics.  Tolerance: none (equality); NaNs are equal."""
+magnitude, near half-way cases, zeros, infinities and NaNs: div_by_normal has
+the bits of `/` on the range that it states and wherever quotient_normal takes
+its result; and its callers on unusual inputs: the pressure solve's divergence,
+the dry thermodynamics and the entropy source of the total-water diffusion.
+Tolerance: none (equality; NaNs are equal) but for the last, 1e-12."""
 import ctypes
 import os
 import subprocess
@@ -11,7 +12,7 @@ import subprocess
 import numpy as np
 import pytest
 
-from helpers import ROOT, gpu_dv, gpu_sim, host_case
+from helpers import ROOT, gpu_dv, gpu_sim, gpu_tends, host_case, oracle_sim, rel_l2
 
 pytestmark = pytest.mark.gpu
 
@@ -20,8 +21,8 @@ PROBE = r"""
 __global__ void probe(const double* a, const double* b, double* q, double* r, double* d, long long n) {
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  q[i] = div_by(a[i], b[i], 1.0 / b[i]);
   r[i] = div_by_normal(a[i], b[i], 1.0 / b[i]);
+  q[i] = quotient_normal(r[i]) ? r[i] : a[i] / b[i];
   d[i] = a[i] / b[i];
 }
 extern "C" int run_probe(const double* a, const double* b, double* q, double* r, double* d, long long n) {
@@ -124,3 +125,48 @@ def test_dry_thermodynamics_of_infinite_entropy(precision):
     d = {n: x.reshape(sim.Gr.shape) for n, x in gpu_dv(sim).items()}
     for n in ("temperature", "alpha", "theta"):
         assert d[n][4, 4, 5] == 0.0 and d[n][5, 4, 7] == np.inf and np.isnan(d[n][6, 6, 6]), n
+
+
+def test_entropy_source_of_dry_and_tiny_vapour(monkeypatch):
+    """Cells without vapour (qv = 0, log of zero) and with qv = 1e-300 beside
+    ordinary ones: the entropy tendency of ScalarDiffusion against the oracle."""
+    import math
+
+    import torch
+    from oracle import port
+    from oracle.sgs import OracleSGS, scheme_from_namelist
+    log = lambda x: math.log(x) if x > 0.0 else (-math.inf if x == 0.0 else math.nan)  # noqa: E731  (as C's)
+    monkeypatch.setattr(port, "_vlog", np.frompyfunc(log, 1, 1))
+    nl, rs, f = host_case(case="bomex", nx=8, ny=7, nz=12)
+    nl = dict(nl, sgs={"scheme": "UniformViscosity", "UniformViscosity": {"diffusivity": 5.0, "viscosity": 5.0}},
+              diffusion={"qt_entropy_source": True})
+    g, o = gpu_sim(nl, rs, f), oracle_sim(nl, rs, f)
+    sh = g.Gr.shape
+    rng = np.random.default_rng(4)
+    o.update_all_bcs()
+    g.PV.Update_all_bcs(g.Gr)
+    o.th_update()
+    g.Th.update(g.Gr, g.RS, g.PV, g.DV)
+    qv = o.dv["qv"].reshape(sh) * (1.0 + 0.1 * rng.standard_normal(sh))
+    qv[4], qv[6] = 0.0, 1e-300
+    o.dv["qv"][:] = qv.ravel()
+    g.DV.get_variable_array("qv", g.Gr).copy_(torch.as_tensor(qv))
+    qt = o.var("qt").reshape(sh)
+    qt *= 1.0 + 0.01 * rng.standard_normal(sh)
+    g.PV.get_variable_array("qt", g.Gr).copy_(torch.as_tensor(qt.copy()))
+    sgs = OracleSGS(scheme_from_namelist(nl), o.d, np.zeros(sh[2]))
+    o.tendencies[:] = 0.0
+    g.PV.tendencies.zero_()
+    with np.errstate(all="ignore"):
+        sgs.ke_update(o)
+        sgs.sgs_update(o)
+        sgs.sd_update(o)
+    g.SGS.update(g.Gr, g.DV, g.PV, g.Ke)
+    g.SD.update(g.Gr, g.RS, g.PV, g.DV)
+    got, want = gpu_tends(g), {n: o.tend(n) for n in ("s", "qt")}
+    for n in ("s", "qt"):
+        a, b = got[n].reshape(sh), want[n].reshape(sh)
+        for x in (np.isnan, np.isposinf, np.isneginf):
+            assert np.array_equal(x(a), x(b)), n
+        ok = np.isfinite(b)
+        assert np.isfinite(b[5]).all() and rel_l2(a[ok], b[ok]) < 1e-12, n
