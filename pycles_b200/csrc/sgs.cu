@@ -43,19 +43,42 @@ struct G {
   double dxi[3];   // DimStruct.dxi (1/dx)
 };
 
-// The row and level of a thread: threads run through the n1 x n2 cells of an
-// x plane, levels fastest, so that only the last block has idle threads
-// (128-thread rows of levels left 106 of 256 idle at 150 levels, in blocks
-// whose registers stayed taken).
-__device__ __forceinline__ bool plane_cell(int n1, int n2, int& j, int& k) {
-  const unsigned p = blockIdx.x * kThreads + threadIdx.x;
-  if (p >= (unsigned)n1 * (unsigned)n2) return false;
-  j = (int)(p / (unsigned)n2);
-  k = (int)(p - (unsigned)j * (unsigned)n2);
-  return true;
+// The plane, row and level of a thread, cells within `margin` of the edges left
+// out.  Flat: threads run through the cells of an x plane, levels fastest, so
+// that only the last block has idle threads (128-thread rows of levels left
+// 106 of 256 idle at 150 levels, in blocks whose registers stayed taken).
+// ROWS: blocks of 128 levels of a row; where these leave few threads idle they
+// are the faster ones (no division, no warp across two rows).  Measured at 160x160 columns, rows and flat: momentum
+// diffusion, 250 levels (2.3% idle) 266 and 268 us, 246 (3.9%) 267 and 265, 112
+// (12%) 134 and 122, 256 (none, the flat map's blocks then are rows) 269 and
+// 268; scalar diffusion of one scalar, 256 levels 80 and 83 us, 250 79 and 82,
+// 246 80 and 81, 240 (6.2%) 80 and 78.
+template <bool ROWS>
+__device__ __forceinline__ bool plane_cell(const G& g, int margin, int& i, int& j, int& k) {
+  if constexpr (ROWS) {
+    k = margin + blockIdx.x * kThreads + threadIdx.x;
+    j = margin + blockIdx.y;
+    i = margin + blockIdx.z;
+    return k < g.n2 - margin;
+  } else {
+    const unsigned n1 = (unsigned)(g.n1 - 2 * margin), n2 = (unsigned)(g.n2 - 2 * margin);
+    const unsigned p = blockIdx.x * kThreads + threadIdx.x;
+    if (p >= n1 * n2) return false;
+    const unsigned q = p / n2;
+    k = margin + (int)(p - q * n2);
+    j = margin + (int)q;
+    i = margin + blockIdx.y;
+    return true;
+  }
 }
-inline dim3 plane_grid(long long n0, long long n1, long long n2) {
-  return dim3((unsigned)((n1 * n2 + kThreads - 1) / kThreads), (unsigned)n0);
+inline dim3 plane_grid(long long n0, long long n1, long long n2, bool rows) {
+  return rows ? dim3((unsigned)((n2 + kThreads - 1) / kThreads), (unsigned)n1, (unsigned)n0)
+              : dim3((unsigned)((n1 * n2 + kThreads - 1) / kThreads), (unsigned)n0);
+}
+// Whether rows of n2 levels leave at most 1/share of the threads idle.
+inline bool rows_fit(long long n2, int share) {
+  const long long lanes = (n2 + kThreads - 1) / kThreads * kThreads;
+  return (lanes - n2) * share <= lanes;
 }
 
 __device__ __forceinline__ long long stride_of(const G& g, int d) { return d == 0 ? g.is : (d == 1 ? g.js : 1); }
@@ -95,9 +118,8 @@ struct KArgs {
 template <int SCHEME, int LENGTH>
 __global__ void __launch_bounds__(kThreads) kinematics_sgs(KArgs a) {
   const G& g = a.g;
-  int j, k;
-  if (!plane_cell(g.n1, g.n2, j, k)) return;
-  const int i = blockIdx.y;
+  int i, j, k;
+  if (!plane_cell<false>(g, 0, i, j, k)) return;
   const long long ijk = (long long)i * g.is + (long long)j * g.js + k;
   double m = 0.0;
   if (i >= 1 && i < g.n0 - 1 && j >= 1 && j < g.n1 - 1 && k >= 1 && k < g.n2 - 1) {
@@ -220,13 +242,11 @@ __device__ __forceinline__ double source_entropy(const SArgs& a, double qt, long
 // (scalar_flux_divergence, Csrc/flux_divergence.h:4-32) and, for qt, the
 // entropy source (compute_qt_diffusion_s_source,
 // Csrc/scalar_diffusion.h:70-113).
+template <bool ROWS>
 __global__ void __launch_bounds__(kThreads, 8) scalar_diffusion(SArgs a) {
   const G& g = a.g;
-  int j, k;
-  if (!plane_cell(g.n1 - 2 * g.gw, g.n2 - 2 * g.gw, j, k)) return;
-  j += g.gw;
-  k += g.gw;
-  const int i = g.gw + blockIdx.y;
+  int i, j, k;
+  if (!plane_cell<ROWS>(g, g.gw, i, j, k)) return;
   const long long ijk = (long long)i * g.is + (long long)j * g.js + k;
   for (int n = 0; n < a.ns; ++n) {
     const double* phi = a.phi[n];
@@ -262,11 +282,8 @@ __global__ void __launch_bounds__(kThreads, 8) scalar_diffusion(SArgs a) {
 template <bool SRC>
 __global__ void __launch_bounds__(kThreads) scalar_diffusion_pair(SArgs a) {
   const G& g = a.g;
-  int j, k;
-  if (!plane_cell(g.n1 - 2 * g.gw, g.n2 - 2 * g.gw, j, k)) return;
-  j += g.gw;
-  k += g.gw;
-  const int i = g.gw + blockIdx.y;
+  int i, j, k;
+  if (!plane_cell<false>(g, g.gw, i, j, k)) return;
   const long long ijk = (long long)i * g.is + (long long)j * g.js + k;
   const double* p0 = a.phi[0];
   const double* p1 = a.phi[1];
@@ -343,16 +360,14 @@ __device__ __forceinline__ double mflux(const MArgs& a, int i1, int i2, long lon
 // entropy source S^2 nu / T (compute_entropy_source,
 // Csrc/momentum_diffusion.h:98-118).
 // Bound by the latency of its L1 loads: 32 registers, so that 64 warps fill an
-// SM (at 38 it took 2.92 ms at 512x512x256 against 2.64).  256x256x256 678 us
-// (672 with rows of 128 levels, which leave no lane idle there), 192x192x150
-// 242 (252), 300x100x101 140 (155).
-__global__ void __launch_bounds__(kThreads, 16) momentum_diffusion(MArgs a) {
+// SM (the flat map at 38 took 2.92 ms at 512x512x256 against 2.64; the row map
+// needs no bound to stay there).  Flat and by rows: 192x192x150 242 and 252 us,
+// 300x100x101 140 and 155.
+template <bool ROWS>
+__global__ void __launch_bounds__(kThreads, ROWS ? 0 : 16) momentum_diffusion(MArgs a) {
   const G& g = a.g;
-  int j, k;
-  if (!plane_cell(g.n1 - 2 * g.gw, g.n2 - 2 * g.gw, j, k)) return;
-  j += g.gw;
-  k += g.gw;
-  const int i = g.gw + blockIdx.y;
+  int i, j, k;
+  if (!plane_cell<ROWS>(g, g.gw, i, j, k)) return;
   const long long ijk = (long long)i * g.is + (long long)j * g.js + k;
   // fully unrolled: the component indices fold into the stencil offsets
   // and the loads shared by the nine fluxes are issued once
@@ -394,7 +409,7 @@ extern "C" int pb_kinematics_sgs(const pb_dims* dims, const pb_sgs* sgs, const d
   if (rc) return rc;
   if (!u || !v || !w || !strain_rate_mag) return PB_ERR_ARG;
   if (dims->nlg[1] > 65535 || dims->nlg[0] > 65535) return PB_ERR_UNSUPPORTED;
-  const dim3 grid = sgsk::plane_grid(dims->nlg[0], dims->nlg[1], dims->nlg[2]);
+  const dim3 grid = sgsk::plane_grid(dims->nlg[0], dims->nlg[1], dims->nlg[2], false);
   cudaStream_t st = as_stream(stream);
   sgsk::KArgs a;
   memset(&a, 0, sizeof(a));
@@ -477,16 +492,19 @@ extern "C" int pb_scalar_diffusion(const pb_dims* dims, const double* rho0, cons
   for (int q = 0; q < 3; ++q) a.dxi_div[q] = 1.0 / dims->dx[q];
   a.qt_index = qt_index;
   a.s_index = qt_index >= 0 ? s_index : -1;
-  const dim3 grid = sgsk::plane_grid(dims->n[0], dims->n[1], dims->n[2]);
+  const bool rows = sgsk::rows_fit(dims->n[2], 24);
   // the usual pair (s, then qt), on four distinct arrays
   const bool pair = nscalars == 2 && (qt_index < 0 || qt_index == 1) && a.tend[0] != a.tend[1] &&
                     a.tend[0] != a.phi[0] && a.tend[0] != a.phi[1] && a.tend[1] != a.phi[0] && a.tend[1] != a.phi[1];
+  const dim3 grid = sgsk::plane_grid(dims->n[0], dims->n[1], dims->n[2], !pair && rows);
   if (pair && qt_index == 1)
     sgsk::scalar_diffusion_pair<true><<<grid, sgsk::kThreads, 0, as_stream(stream)>>>(a);
   else if (pair)
     sgsk::scalar_diffusion_pair<false><<<grid, sgsk::kThreads, 0, as_stream(stream)>>>(a);
+  else if (rows)
+    sgsk::scalar_diffusion<true><<<grid, sgsk::kThreads, 0, as_stream(stream)>>>(a);
   else
-    sgsk::scalar_diffusion<<<grid, sgsk::kThreads, 0, as_stream(stream)>>>(a);
+    sgsk::scalar_diffusion<false><<<grid, sgsk::kThreads, 0, as_stream(stream)>>>(a);
   pb_note_launch();
   PB_LAUNCH_CHECK();
   return PB_OK;
@@ -521,8 +539,12 @@ extern "C" int pb_momentum_diffusion(const pb_dims* dims, const double* rho0, co
   a.tend[1] = vt;
   a.tend[2] = wt;
   a.s_tend = s_tend;
-  const dim3 grid = sgsk::plane_grid(dims->n[0], dims->n[1], dims->n[2]);
-  sgsk::momentum_diffusion<<<grid, sgsk::kThreads, 0, as_stream(stream)>>>(a);
+  const bool rows = sgsk::rows_fit(dims->n[2], 32) && dims->n[2] % sgsk::kThreads != 0;
+  const dim3 grid = sgsk::plane_grid(dims->n[0], dims->n[1], dims->n[2], rows);
+  if (rows)
+    sgsk::momentum_diffusion<true><<<grid, sgsk::kThreads, 0, as_stream(stream)>>>(a);
+  else
+    sgsk::momentum_diffusion<false><<<grid, sgsk::kThreads, 0, as_stream(stream)>>>(a);
   pb_note_launch();
   PB_LAUNCH_CHECK();
   return PB_OK;
