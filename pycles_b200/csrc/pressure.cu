@@ -661,22 +661,29 @@ static int launch_hmean_serial(const Geo& g, const double* w, double* mean, doub
 //     its start (hsum_walk).
 //   * Two more chains start kHmSlack units below and above p.  Rounded
 //     addition is monotone, so a start within kHmSlack / 2 stays between
-//     them; when the two have equal sign and exponent after every addition,
-//     so has everything between.
-//   * Where that does not hold (a sum that starts small and grows, or passes
-//     a power of two or zero within the slack), the walk adds the segment's
-//     columns one by one.  A segment therefore begins at the largest |p|
-//     among the first kHmHead columns around its nominal start: few sums
-//     start small there.  s == p takes the first chain as it is.
+//     them; when the two have equal sign and exponent after an addition, so
+//     has everything between.
+//   * After an addition that leaves the two in different binades (a sum that
+//     cancels: w a wave along y passes zero at the end of every row) the
+//     distances stay as they are if nothing between was rounded: all starts
+//     and the column are multiples of a unit g, and the larger result is below
+//     2^53 g.  g is the unit of the binade that they were in last, and at most
+//     that of the columns added since.
+//   * Where neither holds (a sum that starts small and grows, or passes a
+//     power of two within the slack), the walk adds the segment's columns one
+//     by one.  A segment therefore begins at the largest |p| among the first
+//     kHmHead columns around its nominal start: few sums start small there.
+//     s == p takes the first chain as it is.
 //
 // The walk (one warp per level, ~170 cycles a segment) and the two reads of w
-// bound it.  Measured, FP64 form, one solve: 256x256 columns of 134
-// levels 95 us against 748 for the one-lane chain, 96x96x158 31
-// (108), 64x64x81 21
-// (50).  Segments of 128
-// columns; 64 on grids of up to 8192 columns, where the walk is short and
-// more segments fill the GPU.  Up to 1280 columns hmean_serial stays the
-// faster one (15 us at 32x32 against 20 for the four launches).
+// bound it.  Measured, FP64 form, the mean in one solve: 256x256 columns of
+// 134 levels 95 us against 748 for the one-lane chain, 96x96x158 31 (108),
+// 64x64x81 21 (50).  A whole solve with w a sine along y, where the exact
+// additions count: 64x64x64 90 us, 143 without them (129 with the one-lane
+// chain), 256x256x64 698 (1160, 1153).  Segments of 128 columns; 64 on grids of
+// up to 8192 columns, where the walk is short and more segments fill the GPU.
+// Up to 1280 columns hmean_serial stays the faster one (15 us at 32x32 against
+// 20 for the four launches).
 constexpr int kHmChains = 16;
 constexpr int kHmGrow = 3;  // binades a segment's sums may grow by: 2^(kHmGrow + 1) = kHmChains
 constexpr long long kHmSlack = 1 << 14;
@@ -795,15 +802,22 @@ __global__ void __launch_bounds__(64, 8) hsum_chains(Geo g, const double* __rest
 #pragma unroll
   for (int r = 0; r < kHmChains; ++r) c[r] = from_bits(pb + r);
   double lo = from_bits(pb - kHmSlack), hi = from_bits(pb + kHmSlack);
-  int differ = __double2hiint(lo) ^ __double2hiint(hi);
+  // (without branches, between the additions of the chains)
+  auto sign_exponent = [](double v) { return __double2hiint(v) >> 20; };
+  int unit = sign_exponent(lo) & 0x7ff;  // the exponent whose unit all values are multiples of
+  bool kept = sign_exponent(lo) == sign_exponent(hi);
   int top = 0;  // the largest exponent passed through
   auto add = [&](double v) {
 #pragma unroll
     for (int r = 0; r < kHmChains; ++r) c[r] = add_rn(c[r], v);
     lo = add_rn(lo, v);
     hi = add_rn(hi, v);
-    differ |= __double2hiint(lo) ^ __double2hiint(hi);
-    top = max(top, __double2hiint(hi) & 0x7fffffff);
+    const int l = sign_exponent(lo), h = sign_exponent(hi);
+    const int e = max(l & 0x7ff, h & 0x7ff);
+    const int u = v != 0.0 ? min(unit, sign_exponent(v) & 0x7ff) : unit;
+    kept = kept && (l == h || e <= u);
+    unit = l == h ? e : u;
+    top = max(top, e);
   };
 #pragma unroll
   for (int q = 0; q < kHmHead; ++q) add(q >= b ? x[q] : 0.0);
@@ -825,8 +839,7 @@ __global__ void __launch_bounds__(64, 8) hsum_chains(Geo g, const double* __rest
     for (int q = 0; q + 1 < kHmHead; ++q) add(q < bn ? y[q] : 0.0);
   }
   const int e0 = (int)(pb >> 52) & 0x7ff;
-  top >>= 20;
-  const long long ok = (differ & 0xfff00000) == 0 && top <= e0 + kHmGrow && top < 0x7fe;
+  const long long ok = kept && top <= e0 + kHmGrow && top < 0x7fe;
   double2* row = reinterpret_cast<double2*>(rec + ((long long)k * nsegs + seg) * kHmRow);
 #pragma unroll
   for (int r = 0; r < kHmChains; r += 2) row[r / 2] = make_double2(c[r], c[r + 1]);

@@ -30,6 +30,18 @@ def _columns(kind, n, rng):
         return x * 10.0 ** rng.integers(-12, 12, n)
     if kind == "zeros":
         return np.where(rng.random(n) < 0.9, -0.0, 0.0)
+    if kind == "waves":  # sums that cancel every 64 columns: runs of segments added one by one
+        return np.sin(2.0 * np.pi * np.arange(n) / 64.0)
+    if kind == "returns":  # sums that come back to small values, exactly or nearly, from many binades
+        x *= 2.0 ** rng.integers(-6, 6, n)
+        run = 0.0
+        for i in range(n):
+            if rng.random() < 0.05:
+                x[i] = -float(np.float32(run)) if rng.random() < 0.7 else -run
+            run += x[i]
+        return x
+    if kind == "bursts":  # such runs between segments that move at once
+        return np.where(np.arange(n) // 700 % 2 == 0, np.sin(2.0 * np.pi * np.arange(n) / 64.0), np.abs(x))
     if kind == "tiny":
         return x * 2.0 ** -1060
     if kind == "nonfinite":
@@ -59,3 +71,10 @@ def test_mean_equals_the_serial_chain(grid, kind):
     sim.Pr.solve(Gr, sim.RS, sim.DV, PV)
     got = PV.get_variable_array("w", Gr)[-1].cpu().numpy()
     np.testing.assert_array_equal(got, np.broadcast_to(want, got.shape))
+
+
+@pytest.mark.parametrize("kind", ["waves", "bursts", "returns"])
+@pytest.mark.parametrize("grid", [(41, 64, 5), (64, 64, 3), (90, 91, 3), (96, 101, 6), (128, 130, 3), (150, 64, 28)],
+                         ids=lambda g: "x".join(map(str, g)))
+def test_mean_of_cancelling_columns(grid, kind):
+    test_mean_equals_the_serial_chain(grid, kind)
