@@ -804,22 +804,23 @@ __global__ void __launch_bounds__(64, 8) hsum_chains(Geo g, const double* __rest
 #pragma unroll
   for (int r = 0; r < kHmChains; ++r) c[r] = from_bits(pb + r);
   double lo = from_bits(pb - kHmSlack), hi = from_bits(pb + kHmSlack);
-  // (without branches, between the additions of the chains)
-  auto sign_exponent = [](double v) { return __double2hiint(v) >> 20; };
-  int unit = sign_exponent(lo) & 0x7ff;  // the exponent whose unit all values are multiples of
-  bool kept = sign_exponent(lo) == sign_exponent(hi);
-  int top = 0;  // the largest exponent passed through
+  // (high words, without branches, between the additions of the chains)
+  constexpr int kExp = 0x7ff00000, kMag = 0x7fffffff;
+  int unit = __double2hiint(lo) & kExp;  // the exponent whose unit all values are multiples of
+  bool kept = ((__double2hiint(lo) ^ __double2hiint(hi)) & ~0xfffff) == 0;
+  int top = 0;  // the largest magnitude passed through
   auto add = [&](double v) {
 #pragma unroll
     for (int r = 0; r < kHmChains; ++r) c[r] = add_rn(c[r], v);
     lo = add_rn(lo, v);
     hi = add_rn(hi, v);
-    const int l = sign_exponent(lo), h = sign_exponent(hi);
-    const int e = max(l & 0x7ff, h & 0x7ff);
-    const int u = v != 0.0 ? min(unit, sign_exponent(v) & 0x7ff) : unit;
-    kept = kept && (l == h || e <= u);
-    unit = l == h ? e : u;
-    top = max(top, e);
+    const int l = __double2hiint(lo), h = __double2hiint(hi), hv = __double2hiint(v) & kMag;
+    const int m = max(l & kMag, h & kMag);
+    const bool same = ((l ^ h) & ~0xfffff) == 0;
+    const int u = (hv | __double2loint(v)) != 0 ? min(unit, hv & kExp) : unit;
+    kept = kept && (same || m <= (u | 0xfffff));
+    unit = same ? m & kExp : u;
+    top = max(top, m);
   };
 #pragma unroll
   for (int q = 0; q < kHmHead; ++q) add(q >= b ? x[q] : 0.0);
@@ -841,6 +842,7 @@ __global__ void __launch_bounds__(64, 8) hsum_chains(Geo g, const double* __rest
     for (int q = 0; q + 1 < kHmHead; ++q) add(q < bn ? y[q] : 0.0);
   }
   const int e0 = (int)(pb >> 52) & 0x7ff;
+  top >>= 20;
   const long long ok = kept && top <= e0 + kHmGrow && top < 0x7fe;
   double2* row = reinterpret_cast<double2*>(rec + ((long long)k * nsegs + seg) * kHmRow);
 #pragma unroll
