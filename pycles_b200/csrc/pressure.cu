@@ -973,9 +973,14 @@ constexpr int kDstWrite = 0, kDstAccumulate = 1, kDstDense = 2;
 // correctly rounded, from the reciprocals 1/alpha0_half[k], 1/alpha0[k] and
 // 1/alpha0[k-1] (yh, yf, yd); precision form: multiplications by
 // rho0 = 1/alpha0.
+// `divide` is set if d may differ from the divisions' (divergence_divided): from
+// 2^-500 up to infinity it does not, for an infinity or a NaN among the
+// velocities makes it a NaN here, and quotients too small for div_by_normal
+// (below 2^-900) are absorbed; nor does a smaller d that the sum before it and
+// a dz of that range cancel to.
 template <bool PLAIN>
 __device__ __forceinline__ double divergence_at(const Geo& g, const PArgs& a, long long ijk, long long k, double yh,
-                                                double yf, double yd) {
+                                                double yf, double yd, bool& divide) {
   const double* __restrict__ U = a.u;
   const double* __restrict__ V = a.v;
   const double* __restrict__ Wv = a.w;
@@ -988,24 +993,25 @@ __device__ __forceinline__ double divergence_at(const Geo& g, const PArgs& a, lo
     d = add_rn(d, mul_rn(sub_rn(div_by_normal(V[ijk], ah, yh), div_by_normal(V[ijk - g.js], ah, yh)), g.dxi1));
     const double dz = mul_rn(sub_rn(div_by_normal(wc, a.alpha0[k], yf), div_by_normal(wm, a.alpha0[k - 1], yd)), g.dxi2);
     d = add_rn(d, dz);
-    // From 2^-500 up to infinity d is the divisions' d: an infinity or a NaN
-    // among the velocities makes it a NaN here, and quotients too small for
-    // div_by_normal (below 2^-900) are absorbed; so is a smaller d that the
-    // sum before it and a dz of that range cancel to.  Else: the divisions.
     constexpr unsigned kLow = 0x20b00000u, kInf = 0x7ff00000u;  // high words
     const unsigned td = (unsigned)__double2hiint(d) & 0x7fffffffu, tz = (unsigned)__double2hiint(dz) & 0x7fffffffu;
-    if (!(td - kLow < kInf - kLow || (td < kLow && tz - kLow < kInf - kLow))) {
-      d = 0.0;
-      d = add_rn(d, mul_rn(sub_rn(U[ijk] / ah, U[ijk - g.is] / ah), g.dxi0));
-      d = add_rn(d, mul_rn(sub_rn(V[ijk] / ah, V[ijk - g.js] / ah), g.dxi1));
-      d = add_rn(d, mul_rn(sub_rn(wc / a.alpha0[k], wm / a.alpha0[k - 1]), g.dxi2));
-    }
+    divide |= !((td - kLow < kInf - kLow) | ((td < kLow) & (tz - kLow < kInf - kLow)));
     return d;
   } else {
     const double rh = a.rho0_half[k];
     return (U[ijk] - U[ijk - g.is]) * rh * g.dxi0 + (V[ijk] - V[ijk - g.js]) * rh * g.dxi1 +
            (wc * a.rho0[k] - wm * a.rho0[k - 1]) * g.dxi2;
   }
+}
+
+// The same by divisions.
+__device__ __forceinline__ double divergence_divided(const Geo& g, const PArgs& a, long long ijk, long long k) {
+  const double ah = a.alpha0_half[k];
+  const double wc = sub_rn(a.w[ijk], a.mean[k]), wm = sub_rn(a.w[ijk - 1], a.mean[k - 1]);
+  double d = 0.0;
+  d = add_rn(d, mul_rn(sub_rn(a.u[ijk] / ah, a.u[ijk - g.is] / ah), g.dxi0));
+  d = add_rn(d, mul_rn(sub_rn(a.v[ijk] / ah, a.v[ijk - g.js] / ah), g.dxi1));
+  return add_rn(d, mul_rn(sub_rn(wc / a.alpha0[k], wm / a.alpha0[k - 1]), g.dxi2));
 }
 
 // The refinement residual div - A p of the cell ijk (level k, kk = k - gw),
@@ -1078,6 +1084,7 @@ __global__ void __launch_bounds__((fft_threads<C, LGN>()), (fft_blocks<C, LGN>()
     if ((int)threadIdx.x <= kc) yf[threadIdx.x] = 1.0 / a.alpha0[g.gw + k0 - 1 + threadIdx.x];
     __syncthreads();
   }
+  bool divide = false;
 #pragma unroll 4
   for (int e = threadIdx.x; e < N * KC; e += NT) {
     int kl, il;
@@ -1092,9 +1099,9 @@ __global__ void __launch_bounds__((fft_threads<C, LGN>()), (fft_blocks<C, LGN>()
     double d;
     if constexpr (SRC == kSrcDivergence) {
       if constexpr (PLAIN)
-        d = divergence_at<true>(g, a, ijk, k, yh[kl], yf[kl + 1], yf[kl]);
+        d = divergence_at<true>(g, a, ijk, k, yh[kl], yf[kl + 1], yf[kl], divide);
       else
-        d = divergence_at<false>(g, a, ijk, k, 0.0, 0.0, 0.0);
+        d = divergence_at<false>(g, a, ijk, k, 0.0, 0.0, 0.0, divide);
       div[ijk] = d;
     } else if constexpr (SRC == kSrcResidual) {
       d = residual_at(g, a, ijk, k, k - g.gw, nz);
@@ -1102,6 +1109,22 @@ __global__ void __launch_bounds__((fft_threads<C, LGN>()), (fft_blocks<C, LGN>()
       d = a.src_dense[((long long)il * ny + jl) * nz + k0 + kl];
     }
     inr[slot] = (R)d;
+  }
+  if constexpr (PLAIN) {
+    // a thread's cells once more, where one needs the divisions (a branch in
+    // the loop keeps its loads from running ahead: 11.8 us at 64x64x75, 11.0)
+    if (divide) {
+#pragma unroll 1
+      for (int e = threadIdx.x; e < N * KC; e += NT) {
+        int kl, il;
+        split_idx(e, KC, il, kl);
+        if (kl >= kc) continue;
+        const long long ijk = (g.gw + il) * g.is + j * g.js + g.gw + k0 + kl;
+        const double d = divergence_divided(g, a, ijk, g.gw + k0 + kl);
+        div[ijk] = d;
+        inr[2 * ((kl >> 1) * ld + swz(il)) + (kl & 1)] = d;
+      }
+    }
   }
   __syncthreads();
   const C* res = in;

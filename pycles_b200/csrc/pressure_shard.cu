@@ -36,7 +36,9 @@ __global__ void __launch_bounds__(256) divergence_kernel(Geo g, PArgs a, double*
   const long long ijk = i * g.is + j * g.js + k;
   const double yh = PLAIN ? 1.0 / a.alpha0_half[k] : 0.0;
   const double yf = PLAIN ? 1.0 / a.alpha0[k] : 0.0, yd = PLAIN ? 1.0 / a.alpha0[k - 1] : 0.0;
-  const double d = divergence_at<PLAIN>(g, a, ijk, k, yh, yf, yd);
+  bool divide = false;
+  double d = divergence_at<PLAIN>(g, a, ijk, k, yh, yf, yd, divide);
+  if (PLAIN && divide) d = divergence_divided(g, a, ijk, k);
   a.div[ijk] = d;
   if (dense) dense[((i - g.gw) * ny + (j - g.gw)) * nz + (k - g.gw)] = d;
 }
