@@ -314,11 +314,9 @@ __device__ __forceinline__ void dft_rows(const C* in, C* out, C* table, int nlin
 }
 
 // Any N: G = N / TM rounded up, an index per output.  An output past the last
-// (m = m0 + q G >= N) computes number m - N and is not stored.  Out of line: two
-// forms of it beside dft_rows made the precision form's 150x120x90 solve 1%
-// slower.
+// (m = m0 + q G >= N) computes number m - N and is not stored.
 template <class C, int TM, bool INV>
-__device__ __noinline__ void dft_any(const C* in, C* out, C* stw, int nlines, int N, const C* __restrict__ tw) {
+__device__ __forceinline__ void dft_any(const C* in, C* out, C* stw, int nlines, int N, const C* __restrict__ tw) {
   const int ld = line_ld(N), G = (N + TM - 1) / TM;
   for (int m = threadIdx.x; m < N; m += kFftThreads) {
     C w = tw[m];
@@ -357,32 +355,44 @@ __device__ __noinline__ void dft_any(const C* in, C* out, C* stw, int nlines, in
   __syncthreads();
 }
 
-template <class C, bool INV>
+// The kernels' LGN beside the compile-time lengths: any length, or the few
+// points of dft_any with two outputs (in kernels of its own: beside the others,
+// inlined or called, it changed the allocation of their registers; precision
+// form, one solve of 190x190x40, kernels: 471 us, 479 with it called, 466
+// without; all of dft_any apart: 483).
+constexpr int kFftRuntime = 0, kFftShort = -1;
+
+template <class C, bool INV, bool SHORT>
 __device__ __forceinline__ void dft_lines(const C* in, C* out, C* table, int nlines, int N, int tm,
                                           const C* __restrict__ tw) {
+  if constexpr (SHORT) {
+    dft_any<C, 2, INV>(in, out, table, nlines, N, tw);
+    return;
+  }
   switch (tm) {
     case 4: dft_rows<C, 4, INV>(in, out, table, nlines, N, tw); break;
     case 5: dft_rows<C, 5, INV>(in, out, table, nlines, N, tw); break;
     case 6: dft_rows<C, 6, INV>(in, out, table, nlines, N, tw); break;
     case 8: dft_rows<C, 8, INV>(in, out, table, nlines, N, tw); break;
     case 10: dft_rows<C, 10, INV>(in, out, table, nlines, N, tw); break;
-    case 2: dft_any<C, 2, INV>(in, out, table, nlines, N, tw); break;
     default: dft_any<C, 6, INV>(in, out, table, nlines, N, tw); break;
   }
 }
 
 // Transform the lines in `in`; returns where the result is.
-template <class C>
+template <class C, bool SHORT>
 __device__ __forceinline__ C* fft_lines(C* in, int nlines, int maxlines, int N, const C* __restrict__ tw,
                                         int tm, bool inverse) {
-  if (is_pow2(N)) {
-    fft_lines_pow2<C>(in, nlines, N, tw, inverse);
-    return in;
+  if constexpr (!SHORT) {
+    if (is_pow2(N)) {
+      fft_lines_pow2<C>(in, nlines, N, tw, inverse);
+      return in;
+    }
   }
   C* out = in + (size_t)maxlines * line_ld(N);
   C* table = out + (size_t)maxlines * line_ld(N);
-  if (inverse) dft_lines<C, true>(in, out, table, nlines, N, tm, tw);
-  else dft_lines<C, false>(in, out, table, nlines, N, tm, tw);
+  if (inverse) dft_lines<C, true, SHORT>(in, out, table, nlines, N, tm, tw);
+  else dft_lines<C, false, SHORT>(in, out, table, nlines, N, tm, tw);
   return out;
 }
 
@@ -1041,7 +1051,7 @@ __device__ __forceinline__ double residual_at(const Geo& g, const PArgs& a, long
 //   (a slab of levels of a sharded solve).
 //
 // LGN > 0 instantiates the kernel for N = 2^LGN (KC = 2 ct_lines(LGN)), with
-// the compile-time transform; LGN = 0 takes N and KC at run time.
+// the compile-time transform; the others take N and KC at run time.
 template <class C, int LGN>
 __host__ __device__ constexpr int fft_threads() {
   if constexpr (LGN > 0) return Ct<C, LGN>::NT;
@@ -1052,7 +1062,7 @@ __host__ __device__ constexpr int fft_threads() {
 // three
 template <class C, int LGN>
 constexpr int fft_blocks() {
-  if constexpr (LGN == 0) return sizeof(C) == 16 ? 2 : 3;
+  if constexpr (LGN <= 0) return sizeof(C) == 16 ? 2 : 3;
   return LGN >= 8 ? 2 : 1;
 }
 
@@ -1134,7 +1144,7 @@ __global__ void __launch_bounds__((fft_threads<C, LGN>()), (fft_blocks<C, LGN>()
                                      [&](int l, int x, C v) { in[T::at(l, x)] = v; });
     __syncthreads();
   } else {
-    res = fft_lines<C>(in, lc, KC >> 1, N, twx_of<C>(a), a.tmx, false);
+    res = fft_lines<C, LGN == kFftShort>(in, lc, KC >> 1, N, twx_of<C>(a), a.tmx, false);
   }
   // separate the two rows of each line; write the columns m = 0..N/2
   C* spec = reinterpret_cast<C*>(a.spec);
@@ -1197,7 +1207,7 @@ __global__ void __launch_bounds__((fft_threads<C, LGN>()), (fft_blocks<C, LGN>()
     in[il * ld + swz(jl)] = plane[(long long)jl * Nx + i0 + il];
   }
   __syncthreads();
-  const C* res = fft_lines<C>(in, ic, IC, N, twy_of<C>(a), a.tmy, INV);
+  const C* res = fft_lines<C, LGN == kFftShort>(in, ic, IC, N, twy_of<C>(a), a.tmy, INV);
   const double sc = INV ? 1.0 / (double)N : 1.0;
 #pragma unroll 4
   for (int e = threadIdx.x; e < N * IC; e += kFftThreads) {
@@ -1442,7 +1452,7 @@ __global__ void __launch_bounds__((fft_threads<C, LGN>()), (fft_blocks<C, LGN>()
     }
   }
   __syncthreads();
-  const C* res = fft_lines<C>(in, lc, KC >> 1, N, twx_of<C>(a), a.tmx, true);
+  const C* res = fft_lines<C, LGN == kFftShort>(in, lc, KC >> 1, N, twx_of<C>(a), a.tmx, true);
 #pragma unroll 4
   for (int e = threadIdx.x; e < N * KC; e += kFftThreads) {
     int kl = 0, il = 0;
@@ -1680,7 +1690,7 @@ static int launch_y(const Geo& g, PArgs& a, bool inverse, dim3 grid, size_t sm, 
   return PB_OK;
 }
 
-// Dispatch on a length's compile-time instantiation (LG = 0: run-time length).
+// Dispatch on a length's instantiation (fft_kernel).
 #define PB_FFT_DISPATCH(lg, call)         \
   switch (lg) {                           \
     case 5: { constexpr int L_ = 5; call; } break;   \
@@ -1689,8 +1699,16 @@ static int launch_y(const Geo& g, PArgs& a, bool inverse, dim3 grid, size_t sm, 
     case 8: { constexpr int L_ = 8; call; } break;   \
     case 9: { constexpr int L_ = 9; call; } break;   \
     case 10: { constexpr int L_ = 10; call; } break; \
-    default: { constexpr int L_ = 0; call; } break;  \
+    case kFftShort: { constexpr int L_ = kFftShort; call; } break; \
+    default: { constexpr int L_ = kFftRuntime; call; } break; \
   }
+
+// The kernels of a length: its compile-time ones, those of few points, or those
+// of any length.
+static int fft_kernel(long long n, int tm) {
+  const int lg = ct_lg(n);
+  return lg ? lg : (tm == 2 ? kFftShort : kFftRuntime);
+}
 
 template <class C>
 static size_t ct_smem(int lg) {
@@ -1705,7 +1723,7 @@ static size_t ct_smem(int lg) {
 // y-FFT and inverse x-FFT (to dst).
 struct FftShape {
   long long Nx, Ny, nz, Nh;
-  int LC, KC, IC, lgx, lgy, tmx, tmy;
+  int LC, KC, IC, lgx, lgy, tmx, tmy, kx, ky;
   size_t smx, smy;
   dim3 gx, gy;
 };
@@ -1725,6 +1743,8 @@ static int fft_shape(const Geo& g, FftShape& f) {
   f.smy = f.lgy ? ct_smem<C>(f.lgy) : fft_smem(f.Ny, f.IC, sizeof(C));
   f.tmx = direct_outputs(f.Nx, f.LC, sizeof(C));
   f.tmy = direct_outputs(f.Ny, f.IC, sizeof(C));
+  f.kx = fft_kernel(f.Nx, f.tmx);
+  f.ky = fft_kernel(f.Ny, f.tmy);
   f.gx = dim3((unsigned)f.Ny, ceil_div(f.nz, f.KC));
   f.gy = dim3(ceil_div(f.Nh, f.IC), (unsigned)f.nz);
   return PB_OK;
@@ -1737,11 +1757,11 @@ static int fft_forward(const Geo& g, PArgs& a, int src, cudaStream_t st) {
   if (rc) return rc;
   a.tmx = f.tmx;
   a.tmy = f.tmy;
-  PB_FFT_DISPATCH(f.lgx, rc = (launch_x_fwd<C, L_>(g, a, src, f.gx, f.smx, f.KC, st)));
+  PB_FFT_DISPATCH(f.kx, rc = (launch_x_fwd<C, L_>(g, a, src, f.gx, f.smx, f.KC, st)));
   if (rc) return rc;
   pb_note_launch();
   PB_LAUNCH_CHECK();
-  PB_FFT_DISPATCH(f.lgy, rc = (launch_y<C, L_>(g, a, false, f.gy, f.smy, f.IC, st)));
+  PB_FFT_DISPATCH(f.ky, rc = (launch_y<C, L_>(g, a, false, f.gy, f.smy, f.IC, st)));
   if (rc) return rc;
   pb_note_launch();
   PB_LAUNCH_CHECK();
@@ -1770,11 +1790,11 @@ static int fft_inverse(const Geo& g, PArgs& a, int dst, cudaStream_t st) {
   if (rc) return rc;
   a.tmx = f.tmx;
   a.tmy = f.tmy;
-  PB_FFT_DISPATCH(f.lgy, rc = (launch_y<C, L_>(g, a, true, f.gy, f.smy, f.IC, st)));
+  PB_FFT_DISPATCH(f.ky, rc = (launch_y<C, L_>(g, a, true, f.gy, f.smy, f.IC, st)));
   if (rc) return rc;
   pb_note_launch();
   PB_LAUNCH_CHECK();
-  PB_FFT_DISPATCH(f.lgx, rc = (launch_x_inv<C, L_>(g, a, dst, f.gx, f.smx, f.KC, st)));
+  PB_FFT_DISPATCH(f.kx, rc = (launch_x_inv<C, L_>(g, a, dst, f.gx, f.smx, f.KC, st)));
   if (rc) return rc;
   pb_note_launch();
   PB_LAUNCH_CHECK();
